@@ -1204,6 +1204,375 @@ fd8_ws_kernel(const __grid_constant__ WsMaps maps, T* __restrict__ out, int nx, 
     if (failed && lane == 0) atomicOr(err, ERR_STENCIL_TIMEOUT);
 }
 
+// ---------------------------------------------------------------------------
+// fd8_wq_kernel: the FP32 stencil fed by TMA boxes (the mixed solver's H psi).
+//
+// Same copies as fd8_ws_kernel (a producer warp streams the tile of one plane
+// with its 4-wide x/y halo, wrapped rows and columns as boxes of their own, into
+// a shared ring), but the z derivative is taken from a register queue of INPUTS,
+// so that the sums keep fd8_kernel's order: centre, then the completed x, y and
+// z neighbour sums.  (Pending outputs, as in the FP64 kernels, round at 2^-24 of
+// the ~|c0| partial sums: a 4e-6..6e-6 Ha eigenvalue floor of the mixed solver
+// at h = 0.125 bohr against 8e-7.)
+//
+// A thread owns W x-adjacent points x 2 rows (W = 4 real, 2 complex with both
+// components) and the 9 planes of their z columns in registers.  Step s (output
+// z0 + s) takes the centres of plane s + 8 into the queue and reads the x / y
+// neighbours of plane s + 4 from its stage, so a plane stays in the ring for
+// five steps; S = 8 stages leave three in flight.  V (MODE 1) or the old output
+// (MODE 0) of step s travels with plane s + 8 in a ring of S - 4 slots: slot and
+// stage are both free again after step s.
+// The arithmetic is packed (fma.rn.f32x2 on x pairs): ~17 floating-point
+// instructions per real point instead of 33, which is what the register-prefetch
+// kernel was bound by (issue slots 68 % busy, 122 instructions per point).
+// A warp covers 16 x 16 points (W = 4: 4 quads x 8 row pairs; W = 2: 16 x 8);
+// row pairs are 2 * pitch = 64 (mod 128) bytes apart, so each 128-byte phase of
+// a shared load touches every bank once.  The CTA tile is 16 A x (warp rows) b,
+// A = 2 or 3 compile time (it sets the pitch), b run time: wq_tile() picks them.
+constexpr int WQ_S = 8;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float plo(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float phi(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pk(-1.0f, -1.0f), a); }
+
+// NP pairs (8 NP bytes) from shared memory
+template <int NP>
+__device__ __forceinline__ void lds_pairs(f32x2* v, uint32_t a) {
+    if constexpr (NP == 2)
+        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "r"(a));
+    else
+        asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v[0]) : "r"(a));
+}
+template <int NP>
+__device__ __forceinline__ void stg_pairs(float* p, const f32x2* v) {
+    if constexpr (NP == 2) *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]);
+    else *reinterpret_cast<f32x2*>(p) = v[0];
+}
+
+// packed weights: each fd8 coefficient twice
+struct KQ {
+    f32x2 c0, c0lo;
+    f32x2 cx[4], cy[4], cz[4];
+    f32x2 ax[4], ay[4], az[4];
+};
+
+// Shared-memory layout of a CTA, in bytes (TY: rows of the tile)
+template <bool CPLX, int MODE, int A>
+struct WqLayout {
+    static constexpr int NC = CPLX ? 2 : 1;
+    static constexpr int NE = MODE == 0 ? NC : 1;
+    static constexpr int W = CPLX ? 2 : 4;       // points per thread along x
+    static constexpr int NP = W / 2;             // pairs per row
+    static constexpr int WROWS = CPLX ? 8 : 16;  // rows of one warp
+    static constexpr int TXQ = 16 * A;
+    static constexpr int SW = TXQ + 2 * HW;
+    static constexpr int PITCH = SW * 4;
+    int TY;
+    int main_b, side_b, e_b, stage_b, off_e, off_bar, total;
+    __host__ __device__ explicit WqLayout(int ty) {
+        TY = ty;
+        main_b = (ty + 2 * HW) * PITCH;
+        side_b = ty * HW * 4;
+        e_b = ty * TXQ * 4;
+        stage_b = NC * (main_b + 2 * side_b);
+        off_e = WQ_S * stage_b;
+        off_bar = off_e + (WQ_S - HW) * NE * e_b;
+        total = off_bar + 2 * WQ_S * 8 + 128;
+    }
+};
+
+template <bool CPLX, int MODE, bool GRAD, int A>
+__global__ void __maxnreg__(CPLX ? 168 : 128)
+fd8_wq_kernel(const __grid_constant__ WsMaps maps, float* __restrict__ out, int nx, int ny, int nz, int TY, int zchunk,
+              int nzc, KQ k, int* __restrict__ err) {
+    using LY = WqLayout<CPLX, MODE, A>;
+    constexpr int NC = LY::NC, NE = LY::NE, W = LY::W, NP = LY::NP, TXQ = LY::TXQ, PITCH = LY::PITCH, S = WQ_S;
+    const LY ly(TY);
+    extern __shared__ unsigned char smraw_[];
+    const uint32_t base = (smem_u32(smraw_) + 127u) & ~127u;
+    unsigned char* smraw = smraw_ + (base - smem_u32(smraw_));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smraw + ly.off_bar);
+    uint64_t* empty = full + S;
+    const size_t nxy = (size_t)nx * ny;
+    const size_t N = nxy * nz;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ncw = (int)(blockDim.x >> 5) - 1;      // compute warps
+
+    // work item: tile (x fastest), z chunk, band
+    const int ntx = (nx + TXQ - 1) / TXQ, nty = (ny + TY - 1) / TY;
+    const int tile = blockIdx.x % (ntx * nty), rest = blockIdx.x / (ntx * nty);
+    const int band = rest / nzc;
+    const int x0n = (tile % ntx) * TXQ, y0n = (tile / ntx) * TY;
+    const int x0 = min(x0n, nx - TXQ), y0 = min(y0n, ny - TY);   // loaded tile, inside the grid
+    const bool ledge = x0 == 0, redge = x0 + TXQ == nx;
+    const int z0 = (rest % nzc) * zchunk;
+    const int nsteps = min(nz, z0 + zchunk) - z0;
+    const int nplanes = nsteps + 2 * HW;
+
+    if (threadIdx.x == 0) {
+        for (int st = 0; st < S; ++st) {
+            mbar_init(&full[st], 1);
+            mbar_init(&empty[st], ncw);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+
+    if (warp == ncw) {
+        // ---------------- producer ----------------
+        if (lane != 0) return;
+        const bool yedge = y0 < HW || y0 + TY + HW > ny;
+        const int ytop = y0 - HW < 0 ? y0 - HW + ny : y0 - HW;
+        const int ybot = y0 + TY >= ny ? y0 + TY - ny : y0 + TY;
+        const uint32_t psi_bytes = NC * (ly.main_b + ((ledge ? 1 : 0) + (redge ? 1 : 0)) * ly.side_b);
+        int issued = 0;
+        bool failed = false;
+        for (int j = 0; j < nplanes; ++j) {
+            const int st = j % S;
+            if (j >= S && !mbar_wait(&empty[st], (uint32_t)(((j / S) - 1) & 1))) {
+                failed = true;
+                break;
+            }
+            const bool e_on = j >= 2 * HW;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_expect_tx(&full[st], psi_bytes + (e_on ? NE * ly.e_b : 0));
+            unsigned char* stage = smraw + st * ly.stage_b;
+            const int zz = wrapi(z0 - HW + j, nz);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int zp = (CPLX ? 2 * band + c : band) * nz + zz;
+                unsigned char* mb = stage + c * ly.main_b;
+                if (!yedge) {
+                    tma_load_3d(mb, &maps.full, x0 - HW, y0 - HW, zp, &full[st]);
+                } else {
+                    tma_load_3d(mb, &maps.four, x0 - HW, ytop, zp, &full[st]);
+                    tma_load_3d(mb + HW * PITCH, &maps.body, x0 - HW, y0, zp, &full[st]);
+                    tma_load_3d(mb + (TY + HW) * PITCH, &maps.four, x0 - HW, ybot, zp, &full[st]);
+                }
+#pragma unroll
+                for (int sd = 0; sd < 2; ++sd) {
+                    if (sd == 0 ? !ledge : !redge) continue;
+                    tma_load_3d(stage + NC * ly.main_b + (c * 2 + sd) * ly.side_b, &maps.side, sd == 0 ? nx - HW : 0,
+                                y0, zp, &full[st]);
+                }
+            }
+            if (e_on) {
+                unsigned char* eb = smraw + ly.off_e + (j % (S - HW)) * (NE * ly.e_b);
+#pragma unroll
+                for (int c = 0; c < NE; ++c)
+                    tma_load_3d(eb + c * ly.e_b, &maps.e, x0, y0,
+                                (MODE == 1 ? 0 : (CPLX ? 2 * band + c : band) * nz) + z0 + j - 2 * HW, &full[st]);
+            }
+            issued = j + 1;
+        }
+        if (failed) {
+            atomicOr(err, ERR_STENCIL_TIMEOUT);
+            // copies in flight must land before the CTA may exit
+            for (int st = 0; st < S && st < issued; ++st) {
+                const int last = st + ((issued - 1 - st) / S) * S;
+                (void)mbar_wait(&full[st], (uint32_t)((last / S) & 1));
+            }
+        }
+        return;
+    }
+
+    // ---------------- compute warps ----------------
+    constexpr int LX = 16 / W;                       // lanes along x
+    const int px = (warp % A) * 16 + (lane % LX) * W;             // first point, tile column
+    const int pr = (warp / A) * LY::WROWS + (lane / LX) * 2;      // first row
+    const uint32_t soff = (uint32_t)((pr + HW) * PITCH + (px + HW) * 4);
+    const uint32_t eoff = (uint32_t)(ly.off_e + (pr * TXQ + px) * 4);
+    const bool own0 = x0 + px >= x0n && y0 + pr >= y0n, own1 = x0 + px >= x0n && y0 + pr + 1 >= y0n;
+    float* dst[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+        dst[c] = out + (CPLX ? (size_t)(2 * band + c) : (size_t)band) * N + (size_t)z0 * nxy + (size_t)(x0 + px) +
+                 (size_t)nx * (y0 + pr);
+    // the 4 left / 4 right neighbours of the first row, in pairs of columns:
+    // offset in a stage (component 0), row pitch, component pitch
+    constexpr int NH = 4 / W;                        // loads per side
+    uint32_t xo[2][NH], xr[2][NH], xc[2][NH];
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd)
+#pragma unroll
+        for (int m = 0; m < NH; ++m) {
+            const int cm = sd == 0 ? px + m * W : px + W + HW + m * W;    // column in the main box
+            const bool side = sd == 0 ? ledge && cm < HW : redge && cm >= TXQ + HW;
+            if (side) {
+                xo[sd][m] = (uint32_t)(NC * ly.main_b + sd * ly.side_b +
+                                       (pr * HW + (sd == 0 ? cm : cm - TXQ - HW)) * 4);
+                xr[sd][m] = HW * 4;
+                xc[sd][m] = 2 * ly.side_b;
+            } else {
+                xo[sd][m] = (uint32_t)((pr + HW) * PITCH + cm * 4);
+                xr[sd][m] = PITCH;
+                xc[sd][m] = ly.main_b;
+            }
+        }
+
+    f32x2 q[NC][2][NP][9];
+    bool ok = true;
+    // planes 0..7 fill the queue; the first four are not needed again
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        ok = ok && mbar_wait(&full[j], 0u);
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                f32x2 v[NP];
+                lds_pairs<NP>(v, base + j * ly.stage_b + c * ly.main_b + soff + i * PITCH);
+#pragma unroll
+                for (int h = 0; h < NP; ++h) q[c][i][h][j] = v[h];
+            }
+        if (j < HW) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[j]);
+        }
+    }
+    bool failed = __any_sync(0xffffffffu, !ok);
+
+    for (int sb = 0; sb < nsteps && !failed; sb += 9) {
+#pragma unroll
+        for (int p = 0; p < 9; ++p) {
+            const int s = sb + p;
+            if (s < nsteps && !failed) {
+                const int jn = s + 2 * HW;                         // newest plane
+                if (__any_sync(0xffffffffu, !mbar_wait(&full[jn % S], (uint32_t)((jn / S) & 1)))) {
+                    failed = true;
+                    continue;
+                }
+                const uint32_t nw = base + (uint32_t)(jn % S) * (uint32_t)ly.stage_b;
+                const uint32_t cur = base + (uint32_t)((s + HW) % S) * (uint32_t)ly.stage_b;
+                const uint32_t eb = base + eoff + (uint32_t)(jn % (S - HW)) * (uint32_t)(NE * ly.e_b);
+                f32x2 res[NC][2][NP], grd[NC][2][NP], ev[NE][2][NP];
+#pragma unroll
+                for (int c = 0; c < NE; ++c)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) lds_pairs<NP>(ev[c][i], eb + c * ly.e_b + i * (TXQ * 4));
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const uint32_t sc = cur + c * ly.main_b + soff;
+#define QZ(i, h, kk) q[c][i][h][(p + (kk)) % 9]
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        f32x2 v[NP];
+                        lds_pairs<NP>(v, nw + c * ly.main_b + soff + i * PITCH);
+#pragma unroll
+                        for (int h = 0; h < NP; ++h) QZ(i, h, 8) = v[h];
+                    }
+                    // rows -4..-1 and +2..+5 of the thread's columns (its own two rows are in the queue)
+                    f32x2 col[10][NP];
+#pragma unroll
+                    for (int r = 0; r < 10; ++r) {
+                        if (r == HW || r == HW + 1) {
+#pragma unroll
+                            for (int h = 0; h < NP; ++h) col[r][h] = QZ(r - HW, h, 4);
+                        } else {
+                            lds_pairs<NP>(col[r], sc + (uint32_t)((r - HW) * PITCH));
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        // aligned pairs x-4 .. x+W+3 of the row
+                        f32x2 ap[NP + 4];
+#pragma unroll
+                        for (int m = 0; m < NH; ++m) {
+                            lds_pairs<NP>(&ap[m * NP], cur + xo[0][m] + c * xc[0][m] + i * xr[0][m]);
+                            lds_pairs<NP>(&ap[2 + NP + m * NP], cur + xo[1][m] + c * xc[1][m] + i * xr[1][m]);
+                        }
+#pragma unroll
+                        for (int h = 0; h < NP; ++h) ap[2 + h] = QZ(i, h, 4);
+                        auto at = [&](int n) { return (n & 1) ? phi(ap[n >> 1]) : plo(ap[n >> 1]); };   // x - 4 + n
+#pragma unroll
+                        for (int h = 0; h < NP; ++h) {
+                            const int o = 4 + 2 * h;
+                            const f32x2 ctr = QZ(i, h, 4);
+                            const f32x2 x4 = add2(ap[4 + h], ap[h]), x2 = add2(ap[3 + h], ap[1 + h]);
+                            const f32x2 x3 = pk(at(o + 3) + at(o - 3), at(o + 4) + at(o - 2));
+                            const f32x2 x1 = pk(at(o + 1) + at(o - 1), at(o + 2) + at(o));
+                            // the products in fd8_kernel's contraction order, so that the two agree bit for bit
+                            f32x2 xs = fma2(k.cx[2], x3, mul2(k.cx[3], x4));
+                            xs = fma2(k.cx[1], x2, xs);
+                            xs = fma2(k.cx[0], x1, xs);
+                            f32x2 ys = fma2(k.cy[3], add2(col[i + 8][h], col[i][h]),
+                                            mul2(k.cy[2], add2(col[i + 7][h], col[i + 1][h])));
+                            ys = fma2(k.cy[1], add2(col[i + 6][h], col[i + 2][h]), ys);
+                            ys = fma2(k.cy[0], add2(col[i + 5][h], col[i + 3][h]), ys);
+                            f32x2 zs = fma2(k.cz[3], add2(QZ(i, h, 8), QZ(i, h, 0)),
+                                            mul2(k.cz[2], add2(QZ(i, h, 7), QZ(i, h, 1))));
+                            zs = fma2(k.cz[1], add2(QZ(i, h, 6), QZ(i, h, 2)), zs);
+                            zs = fma2(k.cz[0], add2(QZ(i, h, 5), QZ(i, h, 3)), zs);
+                            f32x2 d = fma2(k.c0, ctr, xs);
+                            d = add2(d, ys);
+                            d = add2(d, zs);
+                            res[c][i][h] = fma2(k.c0lo, ctr, d);
+                            if (GRAD) {
+                                const f32x2 dx4 = sub2(ap[4 + h], ap[h]), dx2 = sub2(ap[3 + h], ap[1 + h]);
+                                const f32x2 dx3 = pk(at(o + 3) - at(o - 3), at(o + 4) - at(o - 2));
+                                const f32x2 dx1 = pk(at(o + 1) - at(o - 1), at(o + 2) - at(o));
+                                f32x2 g = fma2(k.ax[2], dx3, mul2(k.ax[3], dx4));
+                                g = fma2(k.ax[1], dx2, g);
+                                g = fma2(k.ax[0], dx1, g);
+                                f32x2 gy = fma2(k.ay[3], sub2(col[i + 8][h], col[i][h]),
+                                                mul2(k.ay[2], sub2(col[i + 7][h], col[i + 1][h])));
+                                gy = fma2(k.ay[1], sub2(col[i + 6][h], col[i + 2][h]), gy);
+                                gy = fma2(k.ay[0], sub2(col[i + 5][h], col[i + 3][h]), gy);
+                                f32x2 gz = fma2(k.az[3], sub2(QZ(i, h, 8), QZ(i, h, 0)),
+                                                mul2(k.az[2], sub2(QZ(i, h, 7), QZ(i, h, 1))));
+                                gz = fma2(k.az[1], sub2(QZ(i, h, 6), QZ(i, h, 2)), gz);
+                                gz = fma2(k.az[0], sub2(QZ(i, h, 5), QZ(i, h, 3)), gz);
+                                grd[c][i][h] = add2(add2(g, gy), gz);
+                            }
+                        }
+                    }
+#undef QZ
+                }
+                // plane s + 4 and the slot of step s are no longer read
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[(s + HW) % S]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        f32x2 r[NP];
+#pragma unroll
+                        for (int h = 0; h < NP; ++h) {
+                            r[h] = res[c][i][h];
+                            // out.re: Lap(re) - D(im);  out.im: Lap(im) + D(re)
+                            if (CPLX && GRAD) r[h] = c == 0 ? sub2(r[h], grd[NC - 1][i][h]) : add2(r[h], grd[0][i][h]);
+                            r[h] = MODE == 0 ? add2(ev[NE == 1 ? 0 : c][i][h], r[h])
+                                             : fma2(ev[0][i][h], q[c][i][h][(p + 4) % 9], r[h]);
+                        }
+                        if (i == 0 ? own0 : own1) stg_pairs<NP>(dst[c] + (size_t)nx * i + nxy * (size_t)s, r);
+                    }
+                }
+            }
+        }
+    }
+    if (failed && lane == 0) atomicOr(err, ERR_STENCIL_TIMEOUT);
+}
 
 // cuTensorMapEncodeTiled, looked up once through the runtime (no libcuda link)
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1328,6 +1697,95 @@ bool launch_ws(const StencilLaunch& L, const FD8Coef& c, const KC<T>& k, cudaStr
     return true;
 }
 
+// Tile of fd8_wq_kernel for a grid: A (x extent 16 A) and warp rows b, the pair
+// whose tiles copy the fewest bytes through shared memory (points and halo,
+// edge tiles whole), at most 6 compute warps (two or more CTAs per SM).
+// false: no tiling applies (a grid below 32 x 16 points, or one whose halos
+// would straddle the periodic boundary between tiles).
+template <bool CPLX>
+bool wq_tile(int nx, int ny, int* A, int* b) {
+    constexpr int WROWS = CPLX ? 8 : 16;
+    long long best = 0;
+    for (int a = 2; a <= 3; ++a)
+        for (int r = 1; a * r <= 6; ++r) {
+            const int tx = 16 * a, ty = WROWS * r;
+            if (!ws_dim_ok(nx, tx) || !ws_dim_ok(ny, ty)) continue;
+            const long long cost = (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty) *
+                                   ((tx + 2 * HW) * (ty + 2 * HW) + tx * ty);
+            if (best == 0 || cost < best) {
+                best = cost;
+                *A = a;
+                *b = r;
+            }
+        }
+    return best != 0;
+}
+
+template <bool CPLX, int MODE, int A>
+bool launch_wq(const StencilLaunch& L, const FD8Coef& c, const KC<float>& k, int b, cudaStream_t s) {
+    using LY = WqLayout<CPLX, MODE, A>;
+    const LY ly(LY::WROWS * b);
+    const int TY = ly.TY, TXQ = LY::TXQ;
+    const long long planes = (long long)L.nz * L.nb * (CPLX ? 2 : 1);
+    if (planes > (1LL << 31) - 1) return false;
+    WsMaps m;
+    bool ok = make_box_map<float>(&m.full, L.in, L.nx, L.ny, planes, LY::SW, TY + 2 * HW) &&
+              make_box_map<float>(&m.body, L.in, L.nx, L.ny, planes, LY::SW, TY) &&
+              make_box_map<float>(&m.four, L.in, L.nx, L.ny, planes, LY::SW, HW) &&
+              make_box_map<float>(&m.side, L.in, L.nx, L.ny, planes, HW, TY);
+    if (MODE == 1) ok = ok && make_box_map<float>(&m.e, L.V, L.nx, L.ny, L.nz, TXQ, TY);
+    else ok = ok && make_box_map<float>(&m.e, L.out, L.nx, L.ny, planes, TXQ, TY);
+    if (!ok) return false;
+    const bool grad = CPLX && c.has_grad;
+    auto kern = grad ? fd8_wq_kernel<CPLX, MODE, CPLX, A> : fd8_wq_kernel<CPLX, MODE, false, A>;
+    const int threads = (A * b + 1) * 32;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ly.total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, ly.total) != cudaSuccess || per_sm < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    // z chunks: each costs the 8 planes of its halo again, and the last wave of
+    // CTAs is rarely full: the split with the smallest waves x planes
+    const long long tiles = (long long)((L.nx + TXQ - 1) / TXQ) * ((L.ny + TY - 1) / TY);
+    const long long slots = (long long)sm_count() * per_sm;
+    long long best = 0;
+    int zchunk = L.nz;
+    for (int zs = 1; zs <= 8 && L.nz / zs >= 8; ++zs) {
+        const int zc = (L.nz + zs - 1) / zs, n = (L.nz + zc - 1) / zc;
+        const long long cost = ((tiles * n * L.nb + slots - 1) / slots) * (zc + 2 * HW);
+        if (best == 0 || cost < best) {
+            best = cost;
+            zchunk = zc;
+        }
+    }
+    const int nzc = (L.nz + zchunk - 1) / zchunk;
+    const long long items = tiles * nzc * L.nb;
+    if (items > (1LL << 30)) return false;
+    KQ kq;
+    auto two = [](float v) {
+        uint32_t u;
+        std::memcpy(&u, &v, 4);
+        return ((f32x2)u << 32) | u;
+    };
+    kq.c0 = two(k.c0);
+    kq.c0lo = two(k.c0lo);
+    for (int i = 0; i < 4; ++i) {
+        kq.cx[i] = two(k.cx[i]);
+        kq.cy[i] = two(k.cy[i]);
+        kq.cz[i] = two(k.cz[i]);
+        kq.ax[i] = two(k.ax[i]);
+        kq.ay[i] = two(k.ay[i]);
+        kq.az[i] = two(k.az[i]);
+    }
+    kern<<<(unsigned)items, threads, ly.total, s>>>(m, (float*)L.out, L.nx, L.ny, L.nz, TY, zchunk, nzc, kq,
+                                                   device_error_word());
+    return true;
+}
+
 template <typename T, bool CPLX, int MODE, int ZY, int RY, int SREQ, int MINB>
 bool launch_zacc(const StencilLaunch& L, const FD8Coef& c, const KC<T>& k, cudaStream_t s) {
     // ring depth: SREQ stages, or as many as fit MINB CTAs per SM
@@ -1403,6 +1861,12 @@ void launch_t(const StencilLaunch& L, const FD8Coef& c, cudaStream_t s, int vari
                                    : launch_zacc<T, CPLX, MODE, 16, 2, 8, 1>(L, c, k, s);
             if (done) return;
         }
+    }
+    if constexpr (sizeof(T) == 4) {
+        int A = 0, b = 0;
+        if (aligned && pairs_ok && L.tma_ok && variant == 0 && L.nz >= HW && wq_tile<CPLX>(L.nx, L.ny, &A, &b) &&
+            (A == 2 ? launch_wq<CPLX, MODE, 2>(L, c, k, b, s) : launch_wq<CPLX, MODE, 3>(L, c, k, b, s)))
+            return;
     }
     if (CPLX && c.has_grad)
         fd8_kernel<T, CPLX, MODE, CPLX, RY><<<grid, block, 0, s>>>((const T*)L.in, (T*)L.out, (const T*)L.V, L.nx,
