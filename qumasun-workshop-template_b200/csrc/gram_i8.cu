@@ -100,35 +100,80 @@ __device__ __forceinline__ void load4(const T* __restrict__ s, int64_t i, int64_
     }
 }
 
-// maxbits[col] = bits of max_i |u_i,col| (non-negative doubles order like their bits)
+// Four consecutive FP32 elements of a column (zero past N)
+__device__ __forceinline__ float4 load4f(const float* __restrict__ s, int64_t i, int64_t N, bool vec) {
+    if (vec && i + 3 < N) return __ldg(reinterpret_cast<const float4*>(s + i));
+    return make_float4(i < N ? s[i] : 0.0f, i + 1 < N ? s[i + 1] : 0.0f, i + 2 < N ? s[i + 2] : 0.0f,
+                       i + 3 < N ? s[i + 3] : 0.0f);
+}
+
+// maxbits[col] = bits of max_i |u_i,col| as a double (non-negative doubles order
+// like their bits).  Reads the operand once, HBM-bound; FP32 columns are compared
+// in FP32 and only the block's result is converted (the conversion pipe, 16
+// lanes per clock and SM, took twice the read's time).
 template <typename T>
 __global__ void column_absmax_kernel(ColumnSet src, int64_t N, unsigned long long* __restrict__ maxbits) {
     const void* b;
     const int local = column_of(src, blockIdx.y, &b);
     const T* s = static_cast<const T*>(b) + (size_t)local * N;
     const bool vec = ((uintptr_t)s % 16) == 0;
-    double m = 0.0;
+    T m = T(0);
     const int64_t n4 = (N + 3) / 4;
     // unrolled so that several 16-byte loads per thread are in flight
 #pragma unroll 4
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (int64_t)gridDim.x * blockDim.x) {
-        double v[4];
-        load4<T>(s, 4 * q, N, vec, v);
-        m = fmax(m, fmax(fmax(fabs(v[0]), fabs(v[1])), fmax(fabs(v[2]), fabs(v[3]))));
+        if constexpr (sizeof(T) == 4) {
+            const float4 v = load4f(s, 4 * q, N, vec);
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        } else {
+            double v[4];
+            load4<T>(s, 4 * q, N, vec, v);
+            m = fmax(m, fmax(fmax(fabs(v[0]), fabs(v[1])), fmax(fabs(v[2]), fabs(v[3]))));
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    __shared__ double red[32];
+    for (int o = 16; o > 0; o >>= 1) {
+        const T u = __shfl_down_sync(0xffffffffu, m, o);
+        m = m > u ? m : u;
+    }
+    __shared__ T red[32];
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-        atomicMax(&maxbits[blockIdx.y], (unsigned long long)__double_as_longlong(m));
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = m > red[w] ? m : red[w];
+        atomicMax(&maxbits[blockIdx.y], (unsigned long long)__double_as_longlong((double)m));
     }
 }
 
 __device__ __forceinline__ int column_exponent(unsigned long long bits) {
     const double m = __longlong_as_double((long long)bits);
     return m > 0.0 ? ilogb(m) - 5 : 0;   // max |u| 2^-e in [32, 64)
+}
+
+// The four slice words (four int8 each) of four FP32 elements scaled by sa * sb
+// (a power of two).  Every step is exact in FP32: x - rint(x) has no more bits
+// than x, and adding 1.5 * 2^23 rounds to the nearest even integer with that
+// integer's low byte in the sum's own bits.  So the slices are those of the FP64
+// chain below, without its nine conversion-pipe operations per element (16 lanes
+// per clock and SM: they took twice the time of the 8 bytes moved).
+__device__ __forceinline__ void slice4f(float4 v, float sa, float sb, uint32_t (&w)[4]) {
+    constexpr float M = 12582912.0f;   // 1.5 * 2^23
+    float r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        r[j] = __fmul_rn(__fmul_rn(r[j], sa), sb);
+        if (r[j] != r[j]) r[j] = 0.0f;   // a NaN converts to 0 in the FP64 chain
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        uint32_t u[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float t = __fadd_rn(r[j], M);
+            u[j] = __float_as_uint(t);
+            r[j] = __fmul_rn(__fsub_rn(r[j], __fsub_rn(t, M)), 128.0f);
+        }
+        w[k] = __byte_perm(__byte_perm(u[0], u[1], 0x0040), __byte_perm(u[2], u[3], 0x0040), 0x5410);
+    }
 }
 
 // Four int8 slices of column col (length ldk, a multiple of 4; rows N..ldk
@@ -149,6 +194,25 @@ __global__ void slice_kernel(ColumnSet src, int64_t N, int64_t ldk, const unsign
     int8_t* o2 = o0 + 2 * slice_stride;
     int8_t* o3 = o0 + 3 * slice_stride;
     const int64_t n4 = ldk / 4;
+    if constexpr (sizeof(T) == 4) {
+        // -154 <= e <= 122 for finite columns; a column with an infinity (e out of
+        // that range) takes the FP64 chain
+        if (e >= -160 && e <= 126) {
+            const int na = min(-e, 127);
+            const float sa = __uint_as_float((uint32_t)(na + 127) << 23), sb = ldexpf(1.0f, -e - na);
+#pragma unroll 4
+            for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n4;
+                 q += (int64_t)gridDim.x * blockDim.x) {
+                uint32_t w[4];
+                slice4f(load4f(s, 4 * q, N, vec), sa, sb, w);
+                reinterpret_cast<uint32_t*>(o0)[q] = w[0];
+                reinterpret_cast<uint32_t*>(o1)[q] = w[1];
+                reinterpret_cast<uint32_t*>(o2)[q] = w[2];
+                reinterpret_cast<uint32_t*>(o3)[q] = w[3];
+            }
+            return;
+        }
+    }
 #pragma unroll 4
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = 4 * q;
@@ -696,7 +760,9 @@ qsb_status ozaki_split(qsb_dtype dt, int64_t N, const ColumnSet& src, void* dst,
     int* exps = (int*)(w + 4 * stride);
     unsigned long long* maxbits = (unsigned long long*)(w + 4 * stride + a1k((size_t)cols * sizeof(int)));
     QSB_CUDA_TRY(cudaMemsetAsync(maxbits, 0, (size_t)cols * sizeof(unsigned long long), s));
-    const int cblocks = (int)std::min<int64_t>((ldk / 4 + 255) / 256, 256);
+    // about 32 CTAs per SM over all columns: long enough runs per thread for its four loads in
+    // flight (256 CTAs per column gave a thread three or four 16-byte loads in all)
+    const int cblocks = (int)std::min<int64_t>((ldk / 4 + 255) / 256, std::max(1, 4736 / cols));
     if (dt == QSB_F64) {
         column_absmax_kernel<double><<<dim3(cblocks, cols), 256, 0, s>>>(src, N, maxbits);
         slice_kernel<double><<<dim3(cblocks, cols), 256, 0, s>>>(src, N, ldk, maxbits, (int8_t*)w, stride, exps);
