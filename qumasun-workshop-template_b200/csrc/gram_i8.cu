@@ -407,19 +407,25 @@ gram_i8_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ 
 // (2^-27 of the column maxima, below FP32's rounding): near convergence
 // P' = R Cr + P Cp is far smaller than its two terms, and P' and AP' must stay
 // as consistent as FP32 arithmetic keeps them.  The ten products with
-// i + j <= 3 go into four INT32 accumulators (64 output columns per CTA);
-// the epilogue scales by the output column's exponent and stores FP32 planes.
+// i + j <= 3 go into four INT32 accumulators; the epilogue scales by the output
+// column's exponent and stores FP32 planes.
 // ---------------------------------------------------------------------------
-constexpr int RT_K = 128;   // K per stage (rows of the MN-major A tile, bytes of the K-major B rows)
-constexpr int RT_N = 64;    // output columns per CTA (UMMA N)
-constexpr int RT_TILE_B = RT_N * RT_K;          // 8 KB per slice of C'
-constexpr int RT_STAGE_BYTES = 4 * OZ_TILE + 4 * RT_TILE_B;   // four slices of U, four of C'
-// Two stages of the ring of the persistent kernel (one CTA per SM).
-constexpr int RT_STAGES = 2;
-constexpr size_t RT_SMEM = (size_t)RT_STAGES * RT_STAGE_BYTES + 1024 + 256;
+// Column tiles are 128 wide: at 64 (two accumulator sets, the epilogue overlapped
+// with the next tile's MMAs) every row tile's slices crossed L2 -> shared memory
+// four times and each MMA read its A operand for half the columns, 8.1 GB per
+// 96^3 x 384 -> 256 rotation, 1.47 ms; 128 columns move 4.5 GB and leave the
+// readout (all 512 TMEM columns) between two tiles' MMAs: 0.73 ms, most of the
+// difference from the readout's shorter per-element path.
+constexpr int RT_KB = 128;  // K per B stage (bytes of the K-major rows of C')
+constexpr int RT_KA = 64;   // K per A stage (rows of the MN-major A tile): two per B stage
+constexpr int RT_N = 128;   // output columns per tile (UMMA N)
+constexpr int RT_TILE_A = OZ_M * RT_KA;         // 8 KB per slice of U
+constexpr int RT_TILE_B = RT_N * RT_KB;         // 16 KB per slice of C'
+constexpr int RT_SA = 3, RT_SB = 2;             // ring depths
+constexpr size_t RT_SMEM = (size_t)RT_SA * 4 * RT_TILE_A + (size_t)RT_SB * 4 * RT_TILE_B + 1024 + 256;
 static_assert(RT_SMEM <= 232448, "rotation stages must fit the 227 KB of shared memory per CTA");
 
-// kind::i8, A MN-major (bit 15), B K-major, S32 accumulate, M = 128, N = 64
+// kind::i8, A MN-major (bit 15), B K-major, S32 accumulate, M = N = 128
 constexpr uint32_t RT_IDESC = (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(RT_N >> 3) << 17) |
                               ((uint32_t)(OZ_M >> 4) << 24);
 
@@ -444,7 +450,7 @@ __device__ __forceinline__ uint64_t sw128_mnmajor_desc(uint32_t saddr) {
 // [32, 64), four int8 slices, written [j][kpad] (rows K..kpad zero).  One block per column.
 __global__ void rot_coef_split_kernel(const double* __restrict__ C, int ldc, int K, int kpad,
                                       const int* __restrict__ eu, int8_t* __restrict__ slices, size_t stride,
-                                      double* __restrict__ fscale) {
+                                      float* __restrict__ fscale) {
     const int j = blockIdx.x;
     double m = 0.0;
     for (int k = threadIdx.x; k < K; k += blockDim.x) m = fmax(m, fabs(ldexp(C[(size_t)k + (size_t)ldc * j], eu[k])));
@@ -456,7 +462,7 @@ __global__ void rot_coef_split_kernel(const double* __restrict__ C, int ldc, int
     if (threadIdx.x == 0) {
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
         ef = m > 0.0 ? ilogb(m) - 5 : 0;
-        fscale[j] = ldexp(1.0, ef);
+        fscale[j] = (float)(ldexp(1.0, ef) * 0x1p-21);   // units of the four accumulators' exact sum
     }
     __syncthreads();
     const int f = ef;
@@ -483,14 +489,15 @@ __global__ void rot_coef_split_kernel(const double* __restrict__ C, int ldc, int
 }
 
 // Persistent rotation kernel: one CTA per SM walks the output tiles (rows
-// [mt*128, +128) of OUT x columns [nt*64, +64), tile t = mt * ntn + nt, CTAs
+// [mt*128, +128) of OUT x columns [nt*128, +128), tile t = mt * ntn + nt, CTAs
 // take t = blockIdx.x, blockIdx.x + gridDim.x, ...), all of K per tile.
-// Warp 0 lane 0 streams the K stages of every tile into a 2-stage shared
-// ring, warp 1 lane 0 issues the ten MMAs per 32-K step into one of two TMEM
-// accumulator sets (4 x 64 columns each, 512 columns in all), and warps 2-9
-// (two per TMEM lane quarter, 32 output columns each) read a finished set,
-// store it and hand it back -- so the loads of the next
-// stages, the MMAs of the next tile and the epilogue of the last one overlap.
+// Warp 0 lane 0 streams the K stages of every tile into two shared rings (64
+// rows of U per A stage, 128 rows of C' per B stage), warp 1 lane 0 issues the
+// ten MMAs per 32-K step into the four TMEM accumulators (4 x 128 columns), and
+// warps 2-9 (two per TMEM lane quarter, 64 output columns each) read them out,
+// store and hand them back; the loads of the next tile run meanwhile.
+// Column tiles from column zero_col on skip the 128-row blocks of C' that lie in
+// its first zero_rows rows (the caller's zero block: its products are zero).
 // Every wait is bounded: one that runs out sets the device error word and the
 // abort flag; all roles then stop, in-flight copies are drained and TMEM is
 // freed.
@@ -500,32 +507,38 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
 rot_i8_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ CUtensorMap mA1,
               const __grid_constant__ CUtensorMap mA2, const __grid_constant__ CUtensorMap mA3,
               const __grid_constant__ CUtensorMap mB0, const __grid_constant__ CUtensorMap mB1,
-              const __grid_constant__ CUtensorMap mB2, const __grid_constant__ CUtensorMap mB3, int kstages,
-              int64_t N, int q, int ntn, int ntiles, const double* __restrict__ fscale, ColumnSet out,
-              int* __restrict__ err) {
+              const __grid_constant__ CUtensorMap mB2, const __grid_constant__ CUtensorMap mB3, int nka,
+              int zero_rows, int zero_col, int64_t N, int q, int ntn, int ntiles, const float* __restrict__ fscale,
+              ColumnSet out, int* __restrict__ err) {
     extern __shared__ unsigned char rt_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)rt_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)RT_STAGES * RT_STAGE_BYTES);
-    uint64_t* empty = full + RT_STAGES;
-    uint64_t* tfull = empty + RT_STAGES;      // accumulator set ready for the epilogue
-    uint64_t* tempty = tfull + 2;             // accumulator set read out
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    unsigned char* base_b = base + (size_t)RT_SA * 4 * RT_TILE_A;
+    uint64_t* full_a = reinterpret_cast<uint64_t*>(base_b + (size_t)RT_SB * 4 * RT_TILE_B);
+    uint64_t* empty_a = full_a + RT_SA;
+    uint64_t* full_b = empty_a + RT_SA;
+    uint64_t* empty_b = full_b + RT_SB;
+    uint64_t* tfull = empty_b + RT_SB;        // accumulators ready for the epilogue
+    uint64_t* tempty = tfull + 1;             // accumulators read out
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
     int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nk = kstages;
     // tiles of this CTA: t_j = blockIdx.x + j * gridDim.x, j < my_tiles
     const int my_tiles = blockIdx.x < (unsigned)ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    // first A stage (64 rows of K) of column tile nt: an even one, fewer than nka
+    auto first_ka = [&](int nt) { return nt * RT_N >= zero_col ? min(zero_rows / RT_KB, (nka - 1) / 2) * 2 : 0; };
 
     if (threadIdx.x == 0) {
-        for (int st = 0; st < RT_STAGES; ++st) {
-            bar_init(&full[st], 1);
-            bar_init(&empty[st], 1);
+        for (int st = 0; st < RT_SA; ++st) {
+            bar_init(&full_a[st], 1);
+            bar_init(&empty_a[st], 1);
         }
-        for (int b = 0; b < 2; ++b) {
-            bar_init(&tfull[b], 1);
-            bar_init(&tempty[b], 8);
+        for (int st = 0; st < RT_SB; ++st) {
+            bar_init(&full_b[st], 1);
+            bar_init(&empty_b[st], 1);
         }
+        bar_init(tfull, 1);
+        bar_init(tempty, 8);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -540,75 +553,72 @@ rot_i8_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ C
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    int issued = 0;   // stages the producer issued (for the drain)
+    int ga = 0, gb = 0;   // stages the producer issued (for the drain)
     if (warp == 0 && lane == 0) {
         // ---------------- producer ----------------
         const CUtensorMap* amaps[4] = {&mA0, &mA1, &mA2, &mA3};
         const CUtensorMap* bmaps[4] = {&mB0, &mB1, &mB2, &mB3};
-        int g = 0;
-        for (int j = 0; j < my_tiles && !*(volatile int*)abort_flag; ++j) {
+        bool ok = true;
+        for (int j = 0; j < my_tiles && ok; ++j) {
             const int t = (int)blockIdx.x + j * (int)gridDim.x;
             const int mt = t / ntn, nt = t - mt * ntn;
-            for (int it = 0; it < nk; ++it, ++g) {
-                const int st = g % RT_STAGES;
-                if (g >= RT_STAGES && !bar_wait(&empty[st], (uint32_t)(((g / RT_STAGES) - 1) & 1), OZ_WAIT_LIMIT)) {
-                    atomicOr(err, ERR_GEMM_TIMEOUT);
-                    atomicExch(abort_flag, 1);
-                    break;
+            for (int ka = first_ka(nt); ka < nka && ok; ++ka) {
+                if ((ka & 1) == 0) {
+                    const int st = gb % RT_SB;
+                    ok = gb < RT_SB || bar_wait(&empty_b[st], (uint32_t)(((gb / RT_SB) - 1) & 1), OZ_WAIT_LIMIT);
+                    if (ok && !*(volatile int*)abort_flag) {
+                        unsigned char* sp = base_b + (size_t)st * 4 * RT_TILE_B;
+                        bar_expect_tx(&full_b[st], 4 * RT_TILE_B);
+                        // box (128 K, 128 columns of C')
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            tma_2d(sp + k * RT_TILE_B, bmaps[k], (ka / 2) * RT_KB, nt * RT_N, &full_b[st]);
+                        ++gb;
+                    }
                 }
-                if (*(volatile int*)abort_flag) break;
-                unsigned char* sp = base + (size_t)st * RT_STAGE_BYTES;
-                bar_expect_tx(&full[st], RT_STAGE_BYTES);
-                // A: box (128 grid points, 128 columns of U) at (mt*128, it*128); B: box (128 K, 64 columns of C')
-#pragma unroll
-                for (int k = 0; k < 4; ++k) tma_2d(sp + k * OZ_TILE, amaps[k], mt * OZ_M, it * RT_K, &full[st]);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    tma_2d(sp + 4 * OZ_TILE + k * RT_TILE_B, bmaps[k], it * RT_K, nt * RT_N, &full[st]);
-                issued = g + 1;
-            }
-        }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer ----------------
-        int g = 0;
-        for (int j = 0; j < my_tiles && !*(volatile int*)abort_flag; ++j) {
-            const int ab = j & 1;
-            // the epilogue must have read this accumulator set (two tiles ago)
-            if (j >= 2 && !bar_wait(&tempty[ab], (uint32_t)(((j >> 1) - 1) & 1), OZ_WAIT_LIMIT)) {
-                atomicOr(err, ERR_GEMM_TIMEOUT);
-                atomicExch(abort_flag, 1);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t d0 = tmem + (uint32_t)(ab * 4 * RT_N), d1 = d0 + RT_N, d2 = d0 + 2 * RT_N,
-                           d3 = d0 + 3 * RT_N;
-            bool ok = true;
-            for (int it = 0; it < nk; ++it, ++g) {
-                const int st = g % RT_STAGES;
-                if (!bar_wait(&full[st], (uint32_t)((g / RT_STAGES) & 1), OZ_WAIT_LIMIT)) {
+                const int st = ga % RT_SA;
+                ok = ok && (ga < RT_SA || bar_wait(&empty_a[st], (uint32_t)(((ga / RT_SA) - 1) & 1), OZ_WAIT_LIMIT));
+                if (!ok) {
                     atomicOr(err, ERR_GEMM_TIMEOUT);
                     atomicExch(abort_flag, 1);
-                    ok = false;
-                    break;
                 }
                 if (*(volatile int*)abort_flag) {
                     ok = false;
                     break;
                 }
+                unsigned char* sp = base + (size_t)st * 4 * RT_TILE_A;
+                bar_expect_tx(&full_a[st], 4 * RT_TILE_A);
+                // box (128 grid points, 64 columns of U)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) tma_2d(sp + k * RT_TILE_A, amaps[k], mt * OZ_M, ka * RT_KA, &full_a[st]);
+                ++ga;
+            }
+        }
+    } else if (warp == 1 && lane == 0) {
+        // ---------------- MMA issuer ----------------
+        const uint32_t d0 = tmem, d1 = tmem + RT_N, d2 = tmem + 2 * RT_N, d3 = tmem + 3 * RT_N;
+        int ia = 0, ib = 0;
+        bool ok = true;
+        for (int j = 0; j < my_tiles && ok; ++j) {
+            const int t = (int)blockIdx.x + j * (int)gridDim.x;
+            const int k0 = first_ka(t % ntn);
+            // the epilogue must have read the last tile's accumulators
+            ok = j < 1 || bar_wait(tempty, (uint32_t)((j - 1) & 1), OZ_WAIT_LIMIT);
+            for (int ka = k0; ka < nka && ok; ++ka, ++ia) {
+                const int sb = ib % RT_SB, sa = ia % RT_SA;
+                if ((ka & 1) == 0) ok = bar_wait(&full_b[sb], (uint32_t)((ib / RT_SB) & 1), OZ_WAIT_LIMIT);
+                ok = ok && bar_wait(&full_a[sa], (uint32_t)((ia / RT_SA) & 1), OZ_WAIT_LIMIT);
+                if (!ok || *(volatile int*)abort_flag) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t sa = su32(base + (size_t)st * RT_STAGE_BYTES);
-                uint32_t a[4], b[4];
+                const uint32_t pa = su32(base + (size_t)sa * 4 * RT_TILE_A);
+                const uint32_t pb = su32(base_b + (size_t)sb * 4 * RT_TILE_B) + (uint32_t)((ka & 1) * RT_KA);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    a[k] = sa + k * OZ_TILE;
-                    b[k] = sa + 4 * OZ_TILE + k * RT_TILE_B;
-                }
-#pragma unroll
-                for (int kk = 0; kk < RT_K / 32; ++kk) {
+                for (int kk = 0; kk < RT_KA / 32; ++kk) {
                     const uint32_t ao = kk * 4096;   // 32 K rows of 128 bytes (four 8-row atoms)
                     const uint32_t bo = kk * 32;     // 32 int8 along the K-major row
-                    const uint32_t acc = (it > 0 || kk > 0) ? 1u : 0u;
-#define RT_MMA(D, I, J, ACC) umma_i8_mn(D, sw128_mnmajor_desc(a[I] + ao), sw128_kmajor_desc(b[J] + bo), ACC)
+                    const uint32_t acc = (ka > k0 || kk > 0) ? 1u : 0u;
+#define RT_MMA(D, I, J, ACC)                                                                                          \
+    umma_i8_mn(D, sw128_mnmajor_desc(pa + I * RT_TILE_A + ao), sw128_kmajor_desc(pb + J * RT_TILE_B + bo), ACC)
                     RT_MMA(d0, 0, 0, acc);
                     RT_MMA(d1, 0, 1, acc);
                     RT_MMA(d1, 1, 0, 1u);
@@ -621,10 +631,18 @@ rot_i8_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ C
                     RT_MMA(d3, 3, 0, 1u);
 #undef RT_MMA
                 }
-                umma_commit(&empty[st]);
+                umma_commit(&empty_a[sa]);
+                if ((ka & 1) == 1 || ka == nka - 1) {
+                    umma_commit(&empty_b[sb]);
+                    ++ib;
+                }
             }
-            if (!ok) break;
-            umma_commit(&tfull[ab]);
+            if (!ok) {
+                atomicOr(err, ERR_GEMM_TIMEOUT);
+                atomicExch(abort_flag, 1);
+            }
+            if (*(volatile int*)abort_flag) break;
+            umma_commit(tfull);
         }
     } else if (warp >= 2) {
         // ---------------- epilogue (warps 2-9: TMEM lanes 32 (warp % 4) ..., column half (warp - 2) / 4) ----------------
@@ -632,8 +650,7 @@ rot_i8_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ C
         const int chalf = (warp - 2) >> 2;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         for (int j = 0; j < my_tiles; ++j) {
-            const int ab = j & 1;
-            const bool ok = bar_wait(&tfull[ab], (uint32_t)((j >> 1) & 1), OZ_WAIT_LIMIT);
+            const bool ok = bar_wait(tfull, (uint32_t)(j & 1), OZ_WAIT_LIMIT);
             if (!ok) {
                 atomicOr(err, ERR_GEMM_TIMEOUT);
                 atomicExch(abort_flag, 1);
@@ -644,55 +661,63 @@ rot_i8_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ C
             const int t = (int)blockIdx.x + j * (int)gridDim.x;
             const int mt = t / ntn, nt = t - mt * ntn;
             const int64_t gp = (int64_t)mt * OZ_M + quarter * 32 + lane;   // grid point of this TMEM lane
-            const uint32_t dset = tmem + lane_base + (uint32_t)(ab * 4 * RT_N);
-            {
-                const int c0 = chalf * 32;
+#pragma unroll 1
+            for (int ch = 0; ch < 2; ++ch) {
+                const int c0 = chalf * 64 + ch * 32;
                 uint32_t r0[32], r1[32], r2[32], r3[32];
-                tmem_ld32(dset + (uint32_t)c0, r0);
-                tmem_ld32(dset + (uint32_t)(RT_N + c0), r1);
-                tmem_ld32(dset + (uint32_t)(2 * RT_N + c0), r2);
-                tmem_ld32(dset + (uint32_t)(3 * RT_N + c0), r3);
-                if (gp < N && nk > 0) {
+                tmem_ld32(tmem + lane_base + (uint32_t)c0, r0);
+                tmem_ld32(tmem + lane_base + (uint32_t)(RT_N + c0), r1);
+                tmem_ld32(tmem + lane_base + (uint32_t)(2 * RT_N + c0), r2);
+                tmem_ld32(tmem + lane_base + (uint32_t)(3 * RT_N + c0), r3);
+                if (ch == 1) {
+                    // this warp's last values are in registers: hand the accumulators back
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(tempty)) : "memory");
+                }
+                if (gp < N) {
                     const int j0 = nt * RT_N + c0;
+                    // D0 + D1 2^-7 + D2 2^-14 + D3 2^-21 summed exactly as an integer in units of
+                    // 2^-21, one rounding to FP32, then the column's power-of-two scale (exact)
+                    auto value = [&](int jj, float f) {
+                        const long long iv = (long long)(int)r0[jj] * 2097152LL + (long long)(int)r1[jj] * 16384LL +
+                                             (long long)(int)r2[jj] * 128LL + (long long)(int)r3[jj];
+                        return (float)iv * f;
+                    };
                     // one destination lookup for the chunk when its 32 columns lie in one array
+                    // (per-column lookups, bounds and FP64 scales took 53 instructions per
+                    // element: the readout was the longest part of a tile)
                     const void* bp;
                     const int local0 = column_of(out, j0, &bp);
                     const void* bl;
                     const int local31 = j0 + 31 < q ? column_of(out, j0 + 31, &bl) : -1;
-                    const bool one = local31 == local0 + 31 && bl == bp;
-                    float* dst0 = (float*)bp + (size_t)local0 * N + gp;
+                    if (local31 == local0 + 31 && bl == bp) {
+                        float* dst = (float*)bp + (size_t)local0 * N + gp;
 #pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        const int col = j0 + jj;
-                        if (col >= q) continue;
-                        float* dst;
-                        if (one) {
-                            dst = dst0 + (size_t)jj * N;
-                        } else {
+                        for (int jj = 0; jj < 32; ++jj, dst += N) *dst = value(jj, __ldg(fscale + j0 + jj));
+                    } else {
+#pragma unroll
+                        for (int jj = 0; jj < 32; ++jj) {
+                            const int col = j0 + jj;
+                            if (col >= q) continue;
                             const void* bj;
                             const int lj = column_of(out, col, &bj);
-                            dst = (float*)bj + (size_t)lj * N + gp;
+                            ((float*)bj)[(size_t)lj * N + gp] = value(jj, __ldg(fscale + col));
                         }
-                        // D0 + D1 2^-7 + D2 2^-14 + D3 2^-21 summed exactly as an integer in units of
-                        // 2^-21, one rounding to FP32, then the column's power-of-two scale (exact)
-                        const long long iv = (long long)(int)r0[jj] * 2097152LL + (long long)(int)r1[jj] * 16384LL +
-                                             (long long)(int)r2[jj] * 128LL + (long long)(int)r3[jj];
-                        *dst = (float)iv * (float)(__ldg(fscale + col) * 0x1p-21);
                     }
                 }
             }
-            // this warp is done with the set: hand it back to the MMA issuer
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&tempty[ab])) : "memory");
         }
     }
     __syncwarp();
     __syncthreads();
     if (threadIdx.x == 0 && *(volatile int*)abort_flag) {
         // copies in flight must land before the CTA may exit
-        for (int g = max(0, issued - RT_STAGES); g < issued; ++g)
-            (void)bar_wait(&full[g % RT_STAGES], (uint32_t)((g / RT_STAGES) & 1), OZ_DRAIN_LIMIT);
+        for (int g = max(0, ga - RT_SA); g < ga; ++g)
+            (void)bar_wait(&full_a[g % RT_SA], (uint32_t)((g / RT_SA) & 1), OZ_DRAIN_LIMIT);
+        for (int g = max(0, gb - RT_SB); g < gb; ++g)
+            (void)bar_wait(&full_b[g % RT_SB], (uint32_t)((g / RT_SB) & 1), OZ_DRAIN_LIMIT);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -830,32 +855,33 @@ qsb_status gram_ozaki(qsb_dtype dt, int64_t N, int p, int q, const void* U, cons
 }
 
 size_t ozaki_rot_coef_bytes(int K, int q) {
-    const size_t kpad = (size_t)((K + RT_K - 1) / RT_K) * RT_K;
+    const size_t kpad = (size_t)((K + RT_KB - 1) / RT_KB) * RT_KB;
     return 4 * a1k((size_t)q * kpad) + a1k((size_t)q * sizeof(double));
 }
 
 // OUT (fp32 columns, one every N elements, gathered destinations) = U C, with U
 // an ozaki_split operand of K columns and C a K x q FP64 matrix (device, ld ldc).
 // OUT may alias the arrays U was split from: only the slices are read.
+// C's rows [0, zero_rows) are zero in the columns from zero_col on (0: no such block).
 qsb_status ozaki_rotate(int64_t N, const void* Usplit, int K, const double* C, int ldc, int q, const ColumnSet& out,
-                        void* cws, size_t cws_bytes, cudaStream_t s) {
+                        void* cws, size_t cws_bytes, cudaStream_t s, int zero_rows, int zero_col) {
     if (N <= 0 || K <= 0 || q <= 0) return QSB_OK;
     if (column_count(out) != q) return fail(QSB_ERR_INVALID, "ozaki_rotate: output column count");
     if (cws_bytes < ozaki_rot_coef_bytes(K, q)) return fail(QSB_ERR_INVALID, "ozaki_rotate: workspace too small");
-    const int kpad = ((K + RT_K - 1) / RT_K) * RT_K;
+    const int kpad = ((K + RT_KB - 1) / RT_KB) * RT_KB;
     const size_t cstride = a1k((size_t)q * kpad);
     const unsigned char* a = (const unsigned char*)Usplit;
     const size_t sa = oz_stride(N, K);
     const int* eu = (const int*)(a + 4 * sa);
     int8_t* cs = (int8_t*)cws;
-    double* fscale = (double*)((unsigned char*)cws + 4 * cstride);
+    float* fscale = (float*)((unsigned char*)cws + 4 * cstride);
     rot_coef_split_kernel<<<q, 256, 0, s>>>(C, ldc, K, kpad, eu, cs, cstride, fscale);
     QSB_CUDA_TRY(cudaGetLastError());
     const int64_t ldk = oz_ldk(N);
     CUtensorMap m[8];
     for (int k = 0; k < 4; ++k)
-        if (!make_kmajor_map(&m[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a + k * sa, ldk, K, OZ_M, RT_K) ||
-            !make_kmajor_map(&m[4 + k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cs + k * cstride, kpad, q, RT_K, RT_N))
+        if (!make_kmajor_map(&m[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a + k * sa, ldk, K, OZ_M, RT_KA) ||
+            !make_kmajor_map(&m[4 + k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cs + k * cstride, kpad, q, RT_KB, RT_N))
             return fail(QSB_ERR_CUDA, "ozaki_rotate: tensor map encoding failed");
     QSB_CUDA_TRY(cudaFuncSetAttribute(rot_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RT_SMEM));
     const int ntn = (q + RT_N - 1) / RT_N;
@@ -865,8 +891,9 @@ qsb_status ozaki_rotate(int64_t N, const void* Usplit, int K, const double* C, i
     QSB_CUDA_TRY(cudaGetDevice(&dev));
     QSB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int ctas = (int)std::min<long long>(tiles, (long long)sms);
-    rot_i8_kernel<<<ctas, RT_THREADS, RT_SMEM, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], kpad / RT_K, N, q,
-                                                    ntn, (int)tiles, fscale, out, device_error_word());
+    rot_i8_kernel<<<ctas, RT_THREADS, RT_SMEM, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7],
+                                                    (K + RT_KA - 1) / RT_KA, zero_rows, zero_col, N, q, ntn,
+                                                    (int)tiles, fscale, out, device_error_word());
     QSB_CUDA_TRY(cudaGetLastError());
     return QSB_OK;
 }

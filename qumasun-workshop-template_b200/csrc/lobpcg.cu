@@ -832,9 +832,9 @@ qsb_status rotate_real_ozaki(qsb_eigensolver* es, int m, int n, const double* Bs
     normalize_rot_coef<<<n, 256, 0, s>>>(C2, G, m, norms);
     QSB_CUDA_TRY(cudaGetLastError());
     QSB_TRY(ozaki_rotate(es->N, es->su, m, C2, m, 2 * n, column_set(es->X32, n, es->P32, n), es->rotc, es->rotc_bytes,
-                         s));
+                         s, n, n));
     QSB_TRY(ozaki_rotate(es->N, es->sau, m, C2, m, 2 * n, column_set(es->AX32, n, es->AP32, n), es->rotc,
-                         es->rotc_bytes, s));
+                         es->rotc_bytes, s, n, n));
     return QSB_OK;
 }
 

@@ -232,7 +232,7 @@ qsb_status gram_ozaki_tc(int64_t N, const void* A, int p, const void* B, int q, 
 // (device, ld ldc); OUT may alias the arrays U was split from.
 size_t ozaki_rot_coef_bytes(int K, int q);
 qsb_status ozaki_rotate(int64_t N, const void* Usplit, int K, const double* C, int ldc, int q, const ColumnSet& out,
-                        void* cws, size_t cws_bytes, cudaStream_t s);
+                        void* cws, size_t cws_bytes, cudaStream_t s, int zero_rows = 0, int zero_col = 0);
 size_t gram_ozaki_workspace(int64_t N, int p, int q, bool same);
 qsb_status gram_ozaki(qsb_dtype dt, int64_t N, int p, int q, const void* U, const void* V, double* T, int ldt,
                       double alpha, bool accumulate, bool upper, void* ws, size_t ws_bytes, cudaStream_t s);
