@@ -21,9 +21,6 @@
 //    (mCreateNonoverlapList, :3410-3487), and the pull can be fused into the H
 //    stencil so Hpsi is written once.
 #include "qsb_internal.h"
-#include <cstdlib>
-#include <string>
-
 #include <cmath>
 #include <algorithm>
 #include <numeric>
@@ -61,15 +58,62 @@ inline int fold(int v, int n) {
 // ---------------------------------------------------------------------------
 // projection: partial[chunk][w][col] = sum_{p in chunk} beta[p][w] * phi_col[idx_p]
 // phi = psi (real) or psi*exp(+i k.r) (complex; columns 2b = re, 2b+1 = im)
+//
+// The gathers' latency is hidden by an asynchronous pipeline: each thread copies
+// its own points' psi values, beta rows (and coordinates) S - 1 passes ahead into
+// its own slots of a shared ring (cp.async; no thread reads another's slots, so
+// no barrier), which takes no registers.  What bounds it then is the traffic
+// from L2 (~8.8 TB/s for the whole chip, measured, 1.25x the DRAM rate): the
+// beta rows once per CB columns and the sectors at the ends of the sphere's rows.
+// 144^3 x 384 FP32 bands, 54 atoms: 4.69 -> 1.93 ms; 96^3 x 128 FP64, 16 atoms
+// 0.280 -> 0.286 ms (at that bound before).
+// Thread t sums the points t + 256 m in increasing m, then lanes, warps and
+// chunks in order, whatever CB and S are: the mixed-precision solver's results
+// depend on the order of these sums to the bit.
 // ---------------------------------------------------------------------------
-template <typename T, bool CPLX, int WM, int CB, int UP, int MINB>
-__global__ void __launch_bounds__(PROJ_THREADS, MINB)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {
+    static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "cp.async sizes");
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+struct ProjTables {
+    const void* t[4];    // beta and its gradients, [point][wmax]
+    int n;               // how many
+};
+
+template <typename T, bool CPLX, int WM, int CB>
+struct ProjCfg {
+    static constexpr int NCB = CPLX ? 2 * CB : CB;
+    // one point of one thread: psi values, beta rows, coordinates
+    static constexpr int BYTES = NCB * (int)sizeof(T) + WM * (int)sizeof(T) + (CPLX ? 12 : 0);
+    static constexpr int NV = WM * NCB;                      // sums per thread
+    static constexpr int MINB = NV <= 32 ? 2 : 1;            // CTAs per SM (128 / 255 registers)
+    static constexpr int FIT = (MINB == 2 ? 104 : 200) * 1024 / (BYTES * PROJ_THREADS);
+    static constexpr int S = FIT < 2 ? 2 : (FIT > 8 ? 8 : FIT);
+    static constexpr int RING = S * BYTES * PROJ_THREADS;
+    static constexpr int RED = (PROJ_THREADS / 32) * NV * 8;
+    static constexpr int SMEM = RING > RED ? RING : RED;
+    static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
+};
+
+template <typename T, bool CPLX, int WM, int CB>
+__global__ void __launch_bounds__(PROJ_THREADS, (ProjCfg<T, CPLX, WM, CB>::MINB))
 nl_proj_kernel(const int* __restrict__ chunk_order, const int* __restrict__ chunk_begin,
                const int* __restrict__ chunk_end, const int* __restrict__ pt_idx, const int* __restrict__ pt_xyz,
                const T* __restrict__ pt_beta, int wmax, const T* __restrict__ psi, size_t N, int nb, double gx_dx,
                double gy_dy, double gz_dz, double* __restrict__ partial, int ncol) {
-    constexpr int NCB = CPLX ? 2 * CB : CB;
-    constexpr int NV = WM * NCB;
+    using C = ProjCfg<T, CPLX, WM, CB>;
+    constexpr int NCB = C::NCB, S = C::S, NV = C::NV;
+    extern __shared__ __align__(16) unsigned char proj_sm[];
     // launch order: chunks of all atoms by their position along the grid, so
     // that the CTAs in flight together gather from the same region of psi and
     // the overlapping spheres of neighbouring atoms meet in L2; each CTA writes
@@ -78,85 +122,126 @@ nl_proj_kernel(const int* __restrict__ chunk_order, const int* __restrict__ chun
     const int band0 = blockIdx.x * CB;
     const int nbl = min(CB, nb - band0);
     const int p0 = chunk_begin[chunk], p1 = chunk_end[chunk];
+    const int passes = (p1 - p0 + PROJ_THREADS - 1) / PROJ_THREADS;
+    const int t = threadIdx.x;
+
+    // ring layout, per stage: psi [NCB][256] T, beta (rows of 16 bytes [256] when
+    // whole rows can be copied so, else [WM][256] T), coordinates [3][256] int
+    constexpr int STAGE = C::BYTES * PROJ_THREADS;
+    constexpr int BOFF = NCB * (int)sizeof(T) * PROJ_THREADS;
+    constexpr int XOFF = BOFF + WM * (int)sizeof(T) * PROJ_THREADS;
+    constexpr bool VROW = (WM * (int)sizeof(T)) % 16 == 0;
+    constexpr int VPR = VROW ? WM * (int)sizeof(T) / 16 : 1;     // 16-byte pieces of a row
+    const bool vrow = VROW && wmax == WM;
+    const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(proj_sm);
+    const T* psi0 = psi + (size_t)(CPLX ? 2 * band0 : band0) * N;
+
+    auto issue = [&](int m, int idx) {      // copies of this thread's point of pass m
+        const int p = p0 + t + m * PROJ_THREADS;
+        if (p < p1) {
+            const uint32_t st = sm0 + (uint32_t)((m % S) * STAGE);
+#pragma unroll
+            for (int j = 0; j < NCB; ++j)
+                if (j < (CPLX ? 2 * nbl : nbl))
+                    cp_async<(int)sizeof(T)>(st + (uint32_t)((j * PROJ_THREADS + t) * (int)sizeof(T)),
+                                             psi0 + (size_t)j * N + idx);
+            const T* row = pt_beta + (size_t)p * wmax;
+            if (vrow) {
+#pragma unroll
+                for (int v = 0; v < VPR; ++v)
+                    cp_async<16>(st + (uint32_t)(BOFF + (v * PROJ_THREADS + t) * 16), (const char*)row + v * 16);
+            } else {
+#pragma unroll
+                for (int w = 0; w < WM; ++w)
+                    if (w < wmax)
+                        cp_async<(int)sizeof(T)>(st + (uint32_t)(BOFF + (w * PROJ_THREADS + t) * (int)sizeof(T)),
+                                                 row + w);
+            }
+            if (CPLX)
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    cp_async<4>(st + (uint32_t)(XOFF + (d * PROJ_THREADS + t) * 4), pt_xyz + 3 * (size_t)p + d);
+        }
+        cp_commit();
+    };
+    auto index_of = [&](int m) {
+        const int p = p0 + t + m * PROJ_THREADS;
+        return p < p1 ? __ldg(pt_idx + p) : 0;
+    };
 
     double acc[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) acc[i] = 0.0;
-
-    // UP points per thread per pass: their index and psi loads are all issued
-    // before the first use, so UP x CB (x2 complex) gathers are in flight.
-    // Thread t takes the points t + 256 m in increasing m whatever UP is, so
-    // the summation order does not depend on UP.
-    // the grid indices of the next pass are loaded while this pass's psi
-    // gathers are in flight (one dependent load latency per pass, not two)
-    int idx_next[UP];
+    {
+        int idx[S - 1];
 #pragma unroll
-    for (int u = 0; u < UP; ++u) {
-        const int p = p0 + threadIdx.x + u * PROJ_THREADS;
-        idx_next[u] = p < p1 ? __ldg(pt_idx + p) : 0;
+        for (int m = 0; m < S - 1; ++m) idx[m] = index_of(m);
+#pragma unroll
+        for (int m = 0; m < S - 1; ++m) issue(m, idx[m]);
     }
-    for (int pb = p0 + threadIdx.x; pb < p1; pb += PROJ_THREADS * UP) {
-        int idx[UP];
-        bool live[UP];
+    int i0 = index_of(S - 1), i1 = index_of(S);
+    for (int m = 0; m < passes; ++m) {
+        const int i2 = index_of(m + S + 1);
+        issue(m + S - 1, i0);
+        i0 = i1;
+        i1 = i2;
+        cp_wait<S - 1>();
+        const int p = p0 + t + m * PROJ_THREADS;
+        if (p >= p1) continue;
+        const unsigned char* st = proj_sm + (m % S) * STAGE;
+        double b[WM];
+        if (vrow) {
 #pragma unroll
-        for (int u = 0; u < UP; ++u) {
-            live[u] = pb + u * PROJ_THREADS < p1;
-            idx[u] = idx_next[u];
-        }
-        double vals[UP][CPLX ? 2 * CB : CB];
+            for (int v = 0; v < VPR; ++v) {
+                const int4 r = *reinterpret_cast<const int4*>(st + BOFF + (v * PROJ_THREADS + t) * 16);
+                constexpr int E = 16 / (int)sizeof(T);
+                T e[E];
+                memcpy(e, &r, 16);
 #pragma unroll
-        for (int u = 0; u < UP; ++u)
-#pragma unroll
-            for (int j = 0; j < CB; ++j) {
-                const bool ok = live[u] && j < nbl;
-                if (CPLX) {
-                    const size_t base = (size_t)(2 * (band0 + j)) * N;
-                    vals[u][2 * j] = ok ? (double)__ldg(psi + base + idx[u]) : 0.0;
-                    vals[u][2 * j + 1] = ok ? (double)__ldg(psi + base + N + idx[u]) : 0.0;
-                } else {
-                    vals[u][j] = ok ? (double)__ldg(psi + (size_t)(band0 + j) * N + idx[u]) : 0.0;
-                }
+                for (int n = 0; n < E; ++n)
+                    if (v * E + n < WM) b[v * E + n] = (double)e[n];
             }
+        } else {
 #pragma unroll
-        for (int u = 0; u < UP; ++u) {
-            const int p = pb + PROJ_THREADS * UP + u * PROJ_THREADS;
-            idx_next[u] = p < p1 ? __ldg(pt_idx + p) : 0;
+            for (int w = 0; w < WM; ++w)
+                b[w] = w < wmax ? (double)*reinterpret_cast<const T*>(st + BOFF + (w * PROJ_THREADS + t) *
+                                                                                      (int)sizeof(T))
+                                : 0.0;
         }
-#pragma unroll
-        for (int u = 0; u < UP; ++u) {
-            if (!live[u]) continue;
-            const int p = pb + u * PROJ_THREADS;
-            double b[WM];
-#pragma unroll
-            for (int w = 0; w < WM; ++w) b[w] = (w < wmax) ? (double)__ldg(pt_beta + (size_t)p * wmax + w) : 0.0;
+        const T* ps = reinterpret_cast<const T*>(st) + t;
+        if (CPLX) {
+            const int* xs = reinterpret_cast<const int*>(st + XOFF) + t;
+            // mCreateBlochExp (source/PseudoPotNonlocal_SvF2_kpoint.h:3580-3590)
+            const double kxx = gx_dx * (double)xs[0];
+            const double kyy = gy_dy * (double)xs[PROJ_THREADS];
+            const double kzz = gz_dz * (double)xs[2 * PROJ_THREADS];
             double cs = 1.0, sn = 0.0;
-            if (CPLX) {
-                // mCreateBlochExp (source/PseudoPotNonlocal_SvF2_kpoint.h:3580-3590)
-                const double kxx = gx_dx * (double)__ldg(pt_xyz + 3 * (size_t)p + 0);
-                const double kyy = gy_dy * (double)__ldg(pt_xyz + 3 * (size_t)p + 1);
-                const double kzz = gz_dz * (double)__ldg(pt_xyz + 3 * (size_t)p + 2);
-                sincos(kxx + kyy + kzz, &sn, &cs);
-            }
+            sincos(kxx + kyy + kzz, &sn, &cs);
 #pragma unroll
             for (int j = 0; j < CB; ++j) {
-                if (CPLX) {
-                    const double pr = vals[u][2 * j], pi = vals[u][2 * j + 1];
-                    const double fr = cs * pr - sn * pi;   // :4514-4515
-                    const double fi = cs * pi + sn * pr;
+                const double pr = (double)ps[(2 * j) * PROJ_THREADS], pi = (double)ps[(2 * j + 1) * PROJ_THREADS];
+                const double fr = cs * pr - sn * pi;   // :4514-4515
+                const double fi = cs * pi + sn * pr;
 #pragma unroll
-                    for (int w = 0; w < WM; ++w) {
-                        acc[w * NCB + 2 * j] += b[w] * fr;
-                        acc[w * NCB + 2 * j + 1] += b[w] * fi;
-                    }
-                } else {
-#pragma unroll
-                    for (int w = 0; w < WM; ++w) acc[w * NCB + j] += b[w] * vals[u][j];
+                for (int w = 0; w < WM; ++w) {
+                    acc[w * NCB + 2 * j] += b[w] * fr;
+                    acc[w * NCB + 2 * j + 1] += b[w] * fi;
                 }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < CB; ++j) {
+                const double v = (double)ps[j * PROJ_THREADS];
+#pragma unroll
+                for (int w = 0; w < WM; ++w) acc[w * NCB + j] += b[w] * v;
             }
         }
     }
 
-    __shared__ double red[PROJ_THREADS / 32][NV];
+    // block reduction, in the ring's memory once every thread has left the loop
+    cp_wait<0>();
+    __syncthreads();
+    double(*red)[NV] = reinterpret_cast<double(*)[NV]>(proj_sm);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -173,8 +258,215 @@ nl_proj_kernel(const int* __restrict__ chunk_order, const int* __restrict__ chun
         if (jc >= (CPLX ? 2 * nbl : nbl)) continue;
         double s = 0.0;
 #pragma unroll
-        for (int k = 0; k < PROJ_THREADS / 32; ++k) s += red[k][i];
+        for (int q = 0; q < PROJ_THREADS / 32; ++q) s += red[q][i];
         partial[((size_t)chunk * wmax + w) * ncol + col] = s;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The projection as FP64 tensor-core products (mma.m8n8k4; there is no FP64 kind
+// of tcgen05): per chunk, D (projector rows x columns) += B^T (rows x points)
+// psi (points x columns).
+//
+// What bounds it is the traffic from L2 (~8.8 TB/s for the whole chip, measured,
+// 1.25x the DRAM rate): a thread that keeps its own sums (nl_proj_kernel) holds
+// at most 8 columns, so the beta rows cross L2 once per 8 columns, 36 bytes
+// beside 64 of psi.  Here the sums of 8 rows x 8 columns take two registers per
+// lane and the reduction over points happens inside the MMA, so one read of the
+// rows serves NC = 32 columns, or the four tables of the forces (16 rows).
+// The FP64 MMA rate is that of the FP64 pipe; half of the 8 rows are idle at four
+// real projectors, all are used by a complex bundle (beta cos, beta sin) and by
+// the forces.
+//
+// WARPS warps, each with its own batches of 32 points (warp w takes batches w,
+// w + WARPS, ...): the psi values of the next batch are loaded to registers
+// (lanes along points, so the gathers coalesce) while this batch is multiplied
+// from the warp's shared buffer, whose columns lie 36 elements apart, so that a
+// fragment's 4 points x 8 columns touch every bank once.  (cp.async straight to
+// shared memory cost 10 to 18 clocks of the load pipe per 8-byte copy.)  Sums over the
+// batches of a warp in order, then over the warps in order: deterministic.
+// Points past the chunk's end count as zeros.
+// ---------------------------------------------------------------------------
+constexpr int MMA_P = 36;       // elements between columns (rows) of a 32-point batch
+
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// Shared memory of one warp: a batch of psi [NC][36] T, its beta rows [32][rows] T
+// and coordinates [32][3] int, and the A operand [8 MT][36] double
+struct MmaLayout {
+    int beta_off, xyz_off, a_off, warp_bytes;
+    __host__ __device__ MmaLayout(int elem, int NC, int MT, int trows, bool cplx) {
+        beta_off = NC * MMA_P * elem;
+        xyz_off = beta_off + ((32 * trows * elem + 15) / 16) * 16;
+        a_off = xyz_off + (cplx ? 384 : 0);
+        warp_bytes = a_off + 8 * MT * MMA_P * 8;
+    }
+};
+
+// MT: 8-row tiles of the A operand; rows r = table * wmax + w (real), and the
+// same again for the sine parts (complex).  NC: columns per CTA.
+template <typename T, bool CPLX, int MT, int NC, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, (WARPS <= 8 ? 2 : 1))
+nl_proj_mma_kernel(const int* __restrict__ chunk_order, const int* __restrict__ chunk_begin,
+                   const int* __restrict__ chunk_end, const int* __restrict__ pt_idx,
+                   const int* __restrict__ pt_xyz, const ProjTables tabs, int wmax, const T* __restrict__ psi,
+                   size_t N, double gx_dx, double gy_dy, double gz_dz, double* __restrict__ partial,
+                   size_t table_stride, int ncol) {
+    extern __shared__ __align__(16) unsigned char mma_sm[];
+    constexpr int NT = NC / 8;
+    constexpr int TB = (int)sizeof(T);
+    const int trows = tabs.n * wmax;                     // rows without the complex split
+    const MmaLayout ly(TB, NC, MT, trows, CPLX);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* mine = mma_sm + warp * ly.warp_bytes;
+    const uint32_t mine_u = (uint32_t)__cvta_generic_to_shared(mine);
+    double* A = reinterpret_cast<double*>(mine + ly.a_off);
+    const int chunk = chunk_order[blockIdx.y];
+    const int col0 = blockIdx.x * NC;
+    const int ncl = min(NC, ncol - col0);
+    const int p0 = chunk_begin[chunk], p1 = chunk_end[chunk];
+    const int batches = (p1 - p0 + 31) / 32;
+    const T* psi0 = psi + (size_t)col0 * N;
+
+    for (int i = lane; i < 8 * MT * MMA_P; i += 32) A[i] = 0.0;   // rows past the last stay zero
+    auto index_of = [&](int b) {
+        const int p = p0 + 32 * b + lane;
+        return p < p1 ? __ldg(pt_idx + p) : 0;
+    };
+    const bool rows16 = (wmax * TB) % 16 == 0;
+    T v[NC];                                             // psi of the next batch, this lane's point
+    auto load = [&](int b, int idx) {
+        const bool live = p0 + 32 * b + lane < p1;
+        const T* src = psi0 + idx;
+#pragma unroll
+        for (int j = 0; j < NC; ++j, src += N) v[j] = live && j < ncl ? __ldg(src) : T(0);
+    };
+    auto copy_rows = [&](int b) {                        // beta rows and coordinates of batch b
+        const int p = p0 + 32 * b + lane;
+        const size_t pl = (size_t)(p < p1 ? p : p0);
+        for (int k = 0; k < tabs.n; ++k) {
+            const char* row = (const char*)((const T*)tabs.t[k] + pl * wmax);
+            const uint32_t db = mine_u + (uint32_t)(ly.beta_off + (lane * trows + k * wmax) * TB);
+            if (rows16) {
+                for (int o = 0; o < wmax * TB; o += 16) cp_async<16>(db + o, row + o);
+            } else {
+                for (int o = 0; o < wmax * TB; o += TB) cp_async<TB>(db + o, row + o);
+            }
+        }
+        if (CPLX)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                cp_async<4>(mine_u + (uint32_t)(ly.xyz_off + (lane * 3 + d) * 4), pt_xyz + 3 * pl + d);
+        cp_commit();
+    };
+
+    // one column tile: two sums per entry (even and odd fours of points), half the chain of dependent MMAs
+    constexpr int KS = NT == 1 ? 2 : 1;
+    double acc[KS][MT][NT][2];
+#pragma unroll
+    for (int q = 0; q < KS; ++q)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) acc[q][m][n][0] = acc[q][m][n][1] = 0.0;
+
+    int idx = index_of(warp);
+    if (warp < batches) {
+        copy_rows(warp);
+        load(warp, idx);
+    }
+    idx = index_of(warp + WARPS);
+    for (int b = warp; b < batches; b += WARPS) {
+        cp_wait<0>();
+        {
+            T* ps = reinterpret_cast<T*>(mine) + lane;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) ps[j * MMA_P] = v[j];
+        }
+        __syncwarp();
+        const unsigned char* sb = mine;
+        // A operand: this lane's point
+        {
+            const T* br = reinterpret_cast<const T*>(sb + ly.beta_off) + lane * trows;
+            const bool live = p0 + 32 * b + lane < p1;
+            if (CPLX) {
+                const int* xs = reinterpret_cast<const int*>(sb + ly.xyz_off) + lane * 3;
+                // mCreateBlochExp (source/PseudoPotNonlocal_SvF2_kpoint.h:3580-3590)
+                const double kxx = gx_dx * (double)xs[0];
+                const double kyy = gy_dy * (double)xs[1];
+                const double kzz = gz_dz * (double)xs[2];
+                double cs = 1.0, sn = 0.0;
+                sincos(kxx + kyy + kzz, &sn, &cs);
+                for (int r = 0; r < trows; ++r) {
+                    const double v = live ? (double)br[r] : 0.0;
+                    A[r * MMA_P + lane] = v * cs;
+                    A[(trows + r) * MMA_P + lane] = v * sn;
+                }
+            } else {
+                for (int r = 0; r < trows; ++r) A[r * MMA_P + lane] = live ? (double)br[r] : 0.0;
+            }
+        }
+        __syncwarp();
+        if (b + WARPS < batches) {                       // the next batch, in flight during the products
+            copy_rows(b + WARPS);
+            load(b + WARPS, idx);
+        }
+        idx = index_of(b + 2 * WARPS);
+        const T* ps = reinterpret_cast<const T*>(sb) + (lane >> 2) * MMA_P + (lane & 3);
+        const double* as = A + (lane >> 2) * MMA_P + (lane & 3);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            double a[MT];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) a[m] = as[m * 8 * MMA_P + 4 * k];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const double x = (double)ps[n * 8 * MMA_P + 4 * k];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) mma_f64(acc[k % KS][m][n], a[m], x);
+            }
+        }
+        __syncwarp();   // the batch's buffers are free again
+    }
+#pragma unroll
+    for (int q = 1; q < KS; ++q)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) acc[0][m][n][h] += acc[q][m][n][h];
+
+    // sums over the warps, in the buffers' memory once every warp has left the loop
+    cp_wait<0>();
+    __syncthreads();
+    double* red = reinterpret_cast<double*>(mma_sm);     // [warp][8 MT][NC]
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                red[(warp * 8 * MT + m * 8 + (lane >> 2)) * NC + n * 8 + 2 * (lane & 3) + h] = acc[0][m][n][h];
+    __syncthreads();
+    auto total = [&](int r, int c) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) t += red[(q * 8 * MT + r) * NC + c];
+        return t;
+    };
+    for (int i = threadIdx.x; i < trows * NC; i += WARPS * 32) {
+        const int r = i / NC, c = i % NC;
+        if (c >= ncl) continue;
+        double v = total(r, c);
+        // (cos + i sin)(re + i im): re' = cos re - sin im, im' = cos im + sin re (:4514-4515)
+        if (CPLX) v = (c & 1) == 0 ? v - total(trows + r, c + 1) : v + total(trows + r, c - 1);
+        const int k = r / wmax, w = r - k * wmax;
+        partial[k * table_stride + ((size_t)chunk * wmax + w) * ncol + col0 + c] = v;
     }
 }
 
@@ -303,37 +595,104 @@ nl_apply_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restri
 }
 
 // ---------------------------------------------------------------------------
-// expansion, v2: the pull of nl_apply_kernel with the coefficient rows of every
-// atom staged in shared memory one APPLY_CW-column slice at a time (threads
-// whose points share an atom read them as broadcasts instead of per-point L1
-// loads), up to MAXE entries of the point held in registers across all slices,
-// and SG columns of hpsi loaded before use.
+// expansion, pipelined: the pull of nl_apply_kernel with the coefficient rows of
+// the CTA's own atoms (a list made with the tables: the few spheres its 256
+// points lie in, not every atom of the cell) staged in shared memory one
+// APPLY_CW-column slice ahead, up to MAXE entries of the point held in registers
+// for all columns, and hpsi read S - 1 groups of SG columns ahead
+// into the thread's own slots of a shared ring (cp.async).
+// Read-modify-write of hpsi.  Before, every group's loads were issued and waited
+// for in turn and every atom's rows staged by every CTA (2.6 long- and 2.3
+// short-scoreboard stalls per issue, DRAM 25 %); now the load pipe is half busy,
+// with the coefficients' 16-byte loads above all (2.7 passes each where a warp's
+// lanes lie in different spheres), and hpsi moves at 5.0 TB/s (FP64) and 3.2 TB/s
+// (FP32) of the 6.4 a plain read-modify-write reaches.
+// 144^3 x 384 FP32 bands, 54 atoms: 3.37 -> 2.87 ms; 96^3 x 128 bands, 16 atoms:
+// FP32 0.311 -> 0.284, FP64 0.384 -> 0.366 ms.  As FP64 tensor-core products (one
+// coefficient load per 4 x 8 of them) it took 3.08 and 0.456 ms: the accumulator's
+// layout splits every 256-byte row of hpsi into 64-byte pieces.
 // ---------------------------------------------------------------------------
-constexpr int APPLY_CW = 32;
+constexpr int APPLY_CW = 32;    // columns per coefficient slice
+// Real FP64 bundles load a group's hpsi directly, 16 columns at a time (0.366 against 0.388 ms
+// with the ring at 96^3 x 128 bands).
+template <typename T, bool CPLX>
+struct ApplyCfg {
+    static constexpr bool DIRECT = sizeof(T) == 8 && !CPLX;
+    static constexpr int SG = DIRECT ? 16 : 8;               // columns per group
+    // groups in the ring; a slice's copies, issued with the first group of the slice before, are
+    // complete when it starts if S <= groups per slice + 1
+    static constexpr int S = DIRECT ? 0 : (sizeof(T) == 8 ? 3 : 5);
+    static constexpr int RING = S * SG * APPLY_THREADS * (int)sizeof(T);
+    static_assert(S <= APPLY_CW / SG + 1, "a slice must be complete before its first group");
+};
 
-template <typename T, bool CPLX, int WM>
-__global__ void __launch_bounds__(APPLY_THREADS, 2)
-nl_apply2_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restrict__ grid_ptr,
-                 const int* __restrict__ ent_atom, const int* __restrict__ ent_xyz, const T* __restrict__ ent_beta,
-                 int wmax, int n_atoms, const double* __restrict__ coef, int ncol, T* __restrict__ hpsi, size_t N,
-                 double gx_dx, double gy_dy, double gz_dz) {
-    extern __shared__ double csm[];                          // [atom][w][APPLY_CW]
-    constexpr int MAXE = CPLX ? 2 : (WM <= 4 ? 3 : 1);       // entries kept in registers
-    constexpr int SG = CPLX ? 8 : 16;                        // columns per pass
-    const int r = blockIdx.x * APPLY_THREADS + threadIdx.x;
+// doubles of one atom's rows in a slice: 16 bytes of padding keep two atoms' rows in different banks
+__host__ __device__ constexpr int apply_row(int wmax) { return wmax * APPLY_CW + 2; }
+
+// FULL: wmax == WM (no row is padding)
+template <typename T, bool CPLX, int WM, bool FULL>
+__global__ void __launch_bounds__(APPLY_THREADS, (WM <= 4 ? (CPLX || sizeof(T) == 8 ? 2 : 3) : 1))
+nl_apply_ring_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restrict__ grid_ptr,
+                     const int* __restrict__ ent_local, const int* __restrict__ ent_xyz,
+                     const T* __restrict__ ent_beta, int wmax_, const int* __restrict__ cta_ptr,
+                     const int* __restrict__ cta_atoms, int max_local, const double* __restrict__ coef, int ncol,
+                     T* __restrict__ hpsi, size_t N, double gx_dx, double gy_dy, double gz_dz) {
+    const int wmax = FULL ? WM : wmax_;
+    extern __shared__ __align__(16) unsigned char apply_sm[];   // ring [S][SG][256] T, then 2 coefficient slices
+    constexpr int MAXE = WM <= 4 ? 3 : 1;                       // entries kept in registers
+    using CF = ApplyCfg<T, CPLX>;
+    constexpr int SG = CF::SG, S = CF::S;
+    constexpr int STAGE = SG * APPLY_THREADS * (int)sizeof(T);
+    const int arow = apply_row(wmax);
+    double* csm = reinterpret_cast<double*>(apply_sm + CF::RING);
+    const int t = threadIdx.x;
+    const int r = blockIdx.x * APPLY_THREADS + t;
     const bool active = r < n_cov;
+    const int a0 = cta_ptr[blockIdx.x], na = cta_ptr[blockIdx.x + 1] - a0;
+    const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(apply_sm);
+    const uint32_t cm0 = sm0 + (uint32_t)CF::RING;
     int g = 0, e0 = 0, e1 = 0;
     if (active) {
         g = __ldg(cov_grid + r);
         e0 = __ldg(grid_ptr + g);
         e1 = __ldg(grid_ptr + g + 1);
     }
+    T* hp = hpsi + g;
+    // group n: columns [n SG, n SG + SG); its first group also brings slice n SG / CW + 1
+    auto slice = [&](int sl) {
+        const int c0 = sl * APPLY_CW, cw = min(APPLY_CW, ncol - c0);
+        const uint32_t dst = cm0 + (uint32_t)((sl & 1) * max_local * arow * 8);
+        for (int i = t; i < na * wmax * APPLY_CW; i += APPLY_THREADS) {
+            const int k = i % APPLY_CW, aw = i / APPLY_CW, al = aw / wmax, w = aw - al * wmax;
+            if (k < cw)
+                cp_async<8>(dst + (uint32_t)((al * arow + w * APPLY_CW + k) * 8),
+                            coef + ((size_t)__ldg(cta_atoms + a0 + al) * wmax + w) * ncol + c0 + k);
+        }
+    };
+    const int groups = (ncol + SG - 1) / SG;
+    auto issue = [&](int n) {
+        if (!CF::DIRECT && active && n < groups) {
+            const uint32_t dst = sm0 + (uint32_t)((n % (S > 0 ? S : 1)) * STAGE) + (uint32_t)(t * (int)sizeof(T));
+            const T* src = hp + (size_t)(n * SG) * N;
+            const int kc = min(SG, ncol - n * SG);
+#pragma unroll
+            for (int k = 0; k < SG; ++k, src += N)
+                if (k < kc) cp_async<(int)sizeof(T)>(dst + (uint32_t)(k * APPLY_THREADS * (int)sizeof(T)), src);
+        }
+    };
+    slice(0);
+#pragma unroll
+    for (int n = 0; n < S - 1; ++n) {
+        issue(n);
+        cp_commit();
+    }
+
     const int ne = min(MAXE, e1 - e0);
     double b[MAXE][WM];
     int ao[MAXE];
     double cs[MAXE], sn[MAXE];
     auto load_entry = [&](int e, double* bq, int& aq, double& cq, double& sq) {
-        aq = __ldg(ent_atom + e) * wmax * APPLY_CW;
+        aq = __ldg(ent_local + e) * arow;
 #pragma unroll
         for (int w = 0; w < WM; ++w) bq[w] = w < wmax ? (double)__ldg(ent_beta + (size_t)e * wmax + w) : 0.0;
         cq = 1.0;
@@ -358,13 +717,13 @@ nl_apply2_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restr
         }
     }
     // adds entry (bq, aq, phase) times the staged slice to acc[SG]
-    auto contract = [&](const double* bq, int aq, double cq, double sq, int s0, double* acc) {
+    auto contract = [&](const double* sl, const double* bq, int aq, double cq, double sq, int s0, double* acc) {
         if constexpr (!CPLX) {
             // real: no phase, accumulate in place
 #pragma unroll
             for (int w = 0; w < WM; ++w) {
                 if (w < wmax) {
-                    const double* row = csm + aq + w * APPLY_CW + s0;
+                    const double* row = sl + aq + w * APPLY_CW + s0;
 #pragma unroll
                     for (int k = 0; k < SG; k += 2) {
                         const double2 v = *reinterpret_cast<const double2*>(row + k);
@@ -374,22 +733,21 @@ nl_apply2_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restr
                 }
             }
         } else {
-        double tq[SG];
+            double tq[SG];
 #pragma unroll
-        for (int k = 0; k < SG; ++k) tq[k] = 0.0;
+            for (int k = 0; k < SG; ++k) tq[k] = 0.0;
 #pragma unroll
-        for (int w = 0; w < WM; ++w) {
-            if (w < wmax) {
-                const double* row = csm + aq + w * APPLY_CW + s0;
+            for (int w = 0; w < WM; ++w) {
+                if (w < wmax) {
+                    const double* row = sl + aq + w * APPLY_CW + s0;
 #pragma unroll
-                for (int k = 0; k < SG; k += 2) {
-                    const double2 v = *reinterpret_cast<const double2*>(row + k);
-                    tq[k] += bq[w] * v.x;
-                    tq[k + 1] += bq[w] * v.y;
+                    for (int k = 0; k < SG; k += 2) {
+                        const double2 v = *reinterpret_cast<const double2*>(row + k);
+                        tq[k] += bq[w] * v.x;
+                        tq[k + 1] += bq[w] * v.y;
+                    }
                 }
             }
-        }
-        {
             // exp(-i k.r) (source/PseudoPotNonlocal_SvF2_kpoint.h:4026-4027)
 #pragma unroll
             for (int j = 0; j < SG / 2; ++j) {
@@ -397,71 +755,128 @@ nl_apply2_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restr
                 acc[2 * j + 1] += cq * tq[2 * j + 1] - sq * tq[2 * j];
             }
         }
-        }
     };
-    const int slice = n_atoms * wmax * APPLY_CW;
-    for (int c0 = 0; c0 < ncol; c0 += APPLY_CW) {
-        const int cw = min(APPLY_CW, ncol - c0);
-        __syncthreads();   // the previous slice is no longer read
-        for (int i = threadIdx.x; i < slice; i += APPLY_THREADS) {
-            const int k = i % APPLY_CW, aw = i / APPLY_CW;
-            csm[i] = k < cw ? __ldg(coef + (size_t)aw * ncol + c0 + k) : 0.0;
+    for (int n = 0; n < groups; ++n) {
+        const int sl = n / (APPLY_CW / SG);
+        cp_wait<(CF::DIRECT ? 0 : S - 2)>();    // groups up to n have landed (this thread's copies)
+        if (n % (APPLY_CW / SG) == 0) {
+            __syncthreads();                // slice sl is whole, slice sl - 1 is no longer read
+            if ((sl + 1) * APPLY_CW < ncol) slice(sl + 1);
         }
-        __syncthreads();
+        issue(n + S - 1);
+        cp_commit();
         if (!active) continue;
-        for (int s0 = 0; s0 < cw; s0 += SG) {
-            T cur[SG];
+        const int kc = min(SG, ncol - n * SG);
+        T* out = hp + (size_t)(n * SG) * N;
+        T direct[CF::DIRECT ? SG : 1];
+        if constexpr (CF::DIRECT) {
 #pragma unroll
-            for (int k = 0; k < SG; ++k) cur[k] = s0 + k < cw ? hpsi[(size_t)(c0 + s0 + k) * N + g] : T(0);
-            double acc[SG];
-#pragma unroll
-            for (int k = 0; k < SG; ++k) acc[k] = 0.0;
-#pragma unroll
-            for (int q = 0; q < MAXE; ++q)
-                if (q < ne) contract(b[q], ao[q], cs[q], sn[q], s0, acc);
-            // points covered by more than MAXE spheres
-            for (int e = e0 + MAXE; e < e1; ++e) {
-                double bx[WM], cx, sx;
-                int ax;
-                load_entry(e, bx, ax, cx, sx);
-                contract(bx, ax, cx, sx, s0, acc);
-            }
-#pragma unroll
-            for (int k = 0; k < SG; ++k)
-                if (s0 + k < cw) hpsi[(size_t)(c0 + s0 + k) * N + g] = cur[k] + (T)acc[k];
+            for (int k = 0; k < SG; ++k) direct[k] = k < kc ? out[(size_t)k * N] : T(0);
         }
+        const T* cur = reinterpret_cast<const T*>(apply_sm + (n % (S > 0 ? S : 1)) * STAGE) + t;
+        const double* cf = csm + (size_t)(sl & 1) * max_local * arow;
+        const int s0 = n * SG - sl * APPLY_CW;
+        double acc[SG];
+#pragma unroll
+        for (int k = 0; k < SG; ++k) acc[k] = 0.0;
+#pragma unroll
+        for (int q = 0; q < MAXE; ++q)
+            if (q < ne) contract(cf, b[q], ao[q], cs[q], sn[q], s0, acc);
+        // points covered by more than MAXE spheres
+        for (int e = e0 + MAXE; e < e1; ++e) {
+            double bx[WM], cx, sx;
+            int ax;
+            load_entry(e, bx, ax, cx, sx);
+            contract(cf, bx, ax, cx, sx, s0, acc);
+        }
+#pragma unroll
+        for (int k = 0; k < SG; ++k, out += N)
+            if (k < kc) *out = (CF::DIRECT ? direct[CF::DIRECT ? k : 0] : cur[k * APPLY_THREADS]) + (T)acc[k];
     }
+    cp_wait<0>();
 }
 
-// table: -1 projects on beta, 0..2 on the gradient tables d beta / d(x, y, z)
-template <typename T, bool CPLX, int WM>
-void launch_proj(const NLDevice& d, int table, int nb, const void* psi, size_t N, double gx_dx, double gy_dy,
-                 double gz_dz, double* partial, int ncol, cudaStream_t s) {
-    const size_t toff = table < 0 ? 0 : (size_t)table * d.n_points * d.wmax;
-    const T* beta = table < 0 ? (std::is_same<T, double>::value ? (const T*)d.pt_beta64 : (const T*)d.pt_beta32)
-                              : (std::is_same<T, double>::value ? (const T*)d.pt_dbeta64 + toff
-                                                                : (const T*)d.pt_dbeta32 + toff);
-    // up to 4 projectors: 8 real bands (4 complex) x 2 (1) points per thread
-    // in at most 128 registers, two CTAs per SM (at 136 registers, one CTA:
-    // 0.50 ms instead of 0.34 at the 96^3 x 128-band workload; 4 bands x 3
-    // points at 80 registers and three CTAs: 0.35 ms)
-    constexpr int CB = CPLX ? 4 : 8;
-    constexpr int UP = (WM <= 4 && !CPLX) ? 2 : 1;
-    constexpr int MINB = WM <= 4 ? 2 : 1;
-    dim3 grid((nb + CB - 1) / CB, d.n_chunks);
-    nl_proj_kernel<T, CPLX, WM, CB, UP, MINB><<<grid, PROJ_THREADS, 0, s>>>(d.chunk_order, d.chunk_begin, d.chunk_end,
-                                                                        d.pt_idx, d.pt_xyz,
-                                                                        beta, d.wmax, (const T*)psi, N, nb, gx_dx,
-                                                                        gy_dy, gz_dz, partial, ncol);
+template <typename T, bool CPLX, int WM, int CB>
+qsb_status launch_proj(const NLDevice& d, const T* beta, int nb, const void* psi, size_t N, double gx_dx,
+                       double gy_dy, double gz_dz, double* partial, int ncol, cudaStream_t s) {
+    using C = ProjCfg<T, CPLX, WM, CB>;
+    auto kern = nl_proj_kernel<T, CPLX, WM, CB>;
+    QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    const dim3 grid((nb + CB - 1) / CB, d.n_chunks);
+    kern<<<grid, PROJ_THREADS, C::SMEM, s>>>(d.chunk_order, d.chunk_begin, d.chunk_end, d.pt_idx, d.pt_xyz, beta,
+                                             d.wmax, (const T*)psi, N, nb, gx_dx, gy_dy, gz_dz, partial, ncol);
+    QSB_CUDA_TRY(cudaGetLastError());
+    return QSB_OK;
 }
 
+// One table, sums kept per thread
 template <typename T, bool CPLX>
-void launch_proj_w(const NLDevice& d, int table, int nb, const void* psi, size_t N, double gx_dx, double gy_dy,
-                   double gz_dz, double* partial, int ncol, cudaStream_t s) {
-    if (d.wmax <= 1) launch_proj<T, CPLX, 1>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
-    else if (d.wmax <= 4) launch_proj<T, CPLX, 4>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
-    else if (d.wmax <= 9) launch_proj<T, CPLX, 9>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
-    else launch_proj<T, CPLX, 16>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
+qsb_status launch_proj_w(const NLDevice& d, const T* beta, int nb, const void* psi, size_t N, double gx_dx,
+                         double gy_dy, double gz_dz, double* partial, int ncol, cudaStream_t s) {
+    // bands per CTA: 8 real / 4 complex share one read of the beta rows (16 at one CTA per SM:
+    // 0.41 against 0.29 ms, FP64 96^3 x 128); 2 real where
+    // that would leave most SMs without a CTA (few chunks and bands: 18.1 -> 13.1 us for
+    // 12 chunk-groups; a complex point's sincos costs more than the idle SMs)
+    // (half of them at more than 9 projectors: the sums of one thread must fit its registers)
+    constexpr int CB = CPLX ? 4 : 8, CBS = CPLX ? 4 : 2;
+    const bool few = (long long)((nb + CB - 1) / CB) * d.n_chunks < 148;
+#define QSB_PROJ(WM, CBV) \
+    return launch_proj<T, CPLX, WM, CBV>(d, beta, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s)
+    if (few && CBS != CB) {
+        if (d.wmax <= 1) QSB_PROJ(1, CBS);
+        if (d.wmax <= 4) QSB_PROJ(4, CBS);
+    }
+    if (d.wmax <= 1) QSB_PROJ(1, CB);
+    if (d.wmax <= 4) QSB_PROJ(4, CB);
+    if (d.wmax <= 9) QSB_PROJ(9, CB);
+    QSB_PROJ(16, (CB / 2));
+#undef QSB_PROJ
+}
+
+template <typename T, bool CPLX, int MT, int NC, int WARPS>
+qsb_status launch_proj_mma(const NLDevice& d, const ProjTables& tabs, const void* psi, size_t N, double gx_dx,
+                           double gy_dy, double gz_dz, double* partial, size_t table_stride, int ncol,
+                           cudaStream_t s) {
+    auto kern = nl_proj_mma_kernel<T, CPLX, MT, NC, WARPS>;
+    const MmaLayout ly((int)sizeof(T), NC, MT, tabs.n * d.wmax, CPLX);
+    const int smem = std::max(WARPS * ly.warp_bytes, WARPS * 8 * MT * NC * 8);
+    QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const dim3 grid((ncol + NC - 1) / NC, d.n_chunks);
+    kern<<<grid, WARPS * 32, smem, s>>>(d.chunk_order, d.chunk_begin, d.chunk_end, d.pt_idx, d.pt_xyz, tabs,
+                                            d.wmax, (const T*)psi, N, gx_dx, gy_dy, gz_dz, partial, table_stride,
+                                            ncol);
+    QSB_CUDA_TRY(cudaGetLastError());
+    return QSB_OK;
+}
+
+// Tensor-core projection on tabs.n tables, partials of table k at partial + k *
+// table_stride; tabs.n * wmax <= 16.
+template <typename T, bool CPLX>
+qsb_status launch_proj_mma_w(const NLDevice& d, const ProjTables& tabs, const void* psi, size_t N, double gx_dx,
+                             double gy_dy, double gz_dz, double* partial, size_t table_stride, int ncol,
+                             cudaStream_t s) {
+    const int rows = tabs.n * d.wmax * (CPLX ? 2 : 1);
+    // 32 columns per CTA, two CTAs per SM (fewer warps, then columns, as the rows take more
+    // shared memory).  8 columns where fewer CTAs than SMs would come of it, and there with
+    // many warps: the time is then a warp's chain of batches, not bandwidth
+    const int wide = rows <= 16 ? 32 : 16;
+    const bool few = (long long)((ncol + wide - 1) / wide) * d.n_chunks < 148;
+#define QSB_PROJ(MT, NC, WARPS) \
+    return launch_proj_mma<T, CPLX, MT, NC, WARPS>(d, tabs, psi, N, gx_dx, gy_dy, gz_dz, partial, table_stride, ncol, s)
+    if (rows <= 8) {
+        if (few) QSB_PROJ(1, 8, 32);
+        QSB_PROJ(1, 32, 8);
+    }
+    if (rows <= 16) {
+        if (few) QSB_PROJ(2, 8, 16);
+        QSB_PROJ(2, 32, 6);
+    }
+    if constexpr (CPLX) {
+        if (few) QSB_PROJ(4, 8, 12);
+        QSB_PROJ(4, 16, 6);
+    }
+#undef QSB_PROJ
+    return fail(QSB_ERR_INVALID, "nonlocal: more than 16 projector rows");
 }
 
 // Per atom (one block): energy = sum over bands and projectors of occ E_w |c|^2;
@@ -509,10 +924,10 @@ void nl_free(NLDevice& d) {
     dfree(d.atom_width); dfree(d.atom_proj_off); dfree(d.atom_E);
     dfree(d.chunk_atom); dfree(d.chunk_begin); dfree(d.chunk_end); dfree(d.chunk_order);
     dfree(d.atom_chunk_begin); dfree(d.atom_chunk_end);
-    dfree(d.grid_ptr); dfree(d.cov_grid); dfree(d.ent_atom); dfree(d.ent_xyz);
+    dfree(d.grid_ptr); dfree(d.cov_grid); dfree(d.ent_atom); dfree(d.ent_local); dfree(d.cta_ptr); dfree(d.cta_atoms); dfree(d.ent_xyz);
     dfree(d.ent_beta64); dfree(d.ent_beta32);
     dfree(d.pt_dbeta64); dfree(d.pt_dbeta32);
-    d.n_atoms = 0; d.wmax = 0; d.n_points = 0; d.total_proj = 0; d.n_chunks = 0; d.n_cov = 0;
+    d.n_atoms = 0; d.wmax = 0; d.n_points = 0; d.total_proj = 0; d.n_chunks = 0; d.n_cov = 0; d.max_local = 0;
     d.h_atom_width.clear(); d.h_atom_proj_off.clear(); d.h_npts.clear(); d.h_src.clear();
 }
 
@@ -617,6 +1032,31 @@ qsb_status nl_upload(NLDevice& d, int nx, int ny, int nz, int n_atoms, const int
         if (gptr[g + 1] > gptr[g]) cov.push_back((int)g);
     d.n_cov = (int)cov.size();
 
+    // atoms of each run of APPLY_THREADS covered points (one CTA of the expansion), ascending,
+    // and every entry's place in its run's list
+    std::vector<int> cptr(1, 0), catoms, e_local(total);
+    d.max_local = 0;
+    {
+        std::vector<int> seen(n_atoms, -1), here;
+        for (size_t r0 = 0; r0 < cov.size(); r0 += APPLY_THREADS) {
+            const size_t r1 = std::min(cov.size(), r0 + (size_t)APPLY_THREADS);
+            here.clear();
+            for (size_t r = r0; r < r1; ++r)
+                for (int e = gptr[cov[r]]; e < gptr[cov[r] + 1]; ++e)
+                    if (seen[e_atom[e]] != (int)r0) {
+                        seen[e_atom[e]] = (int)r0;
+                        here.push_back(e_atom[e]);
+                    }
+            std::sort(here.begin(), here.end());
+            for (size_t r = r0; r < r1; ++r)
+                for (int e = gptr[cov[r]]; e < gptr[cov[r] + 1]; ++e)
+                    e_local[e] = (int)(std::lower_bound(here.begin(), here.end(), e_atom[e]) - here.begin());
+            catoms.insert(catoms.end(), here.begin(), here.end());
+            cptr.push_back((int)catoms.size());
+            d.max_local = std::max(d.max_local, (int)here.size());
+        }
+    }
+
     std::vector<float> b32(b64.begin(), b64.end()), e_b32(e_b64.begin(), e_b64.end());
     QSB_TRY(dupload(d.pt_idx, idx.data(), idx.size()));
     QSB_TRY(dupload(d.pt_xyz, xyz.data(), xyz.size()));
@@ -634,6 +1074,9 @@ qsb_status nl_upload(NLDevice& d, int nx, int ny, int nz, int n_atoms, const int
     QSB_TRY(dupload(d.grid_ptr, gptr.data(), gptr.size()));
     QSB_TRY(dupload(d.cov_grid, cov.data(), cov.size()));
     QSB_TRY(dupload(d.ent_atom, e_atom.data(), e_atom.size()));
+    QSB_TRY(dupload(d.ent_local, e_local.data(), e_local.size()));
+    QSB_TRY(dupload(d.cta_ptr, cptr.data(), cptr.size()));
+    QSB_TRY(dupload(d.cta_atoms, catoms.data(), catoms.size()));
     QSB_TRY(dupload(d.ent_xyz, e_xyz.data(), e_xyz.size()));
     QSB_TRY(dupload(d.ent_beta64, e_b64.data(), e_b64.size()));
     QSB_TRY(dupload(d.ent_beta32, e_b32.data(), e_b32.size()));
@@ -648,27 +1091,48 @@ size_t nl_workspace_bytes(const NLDevice& d, int ncol) {
 }
 
 namespace {
-qsb_status nl_project_table(qsb_dtype dt, const NLDevice& d, int table, int nx, int ny, int nz, int nb,
-                            int is_complex, const void* psi, double dV, double gx_dx, double gy_dy, double gz_dz,
-                            bool inner_only, void* ws, double** coef_out, cudaStream_t s) {
+// coef_out[k] of table first_table + k (-1: beta, 0..2: the gradient tables), each
+// table with its own partials and coefficients in ws (nl_workspace_bytes apart)
+qsb_status nl_project_tables(qsb_dtype dt, const NLDevice& d, int first_table, int ntab, int nx, int ny, int nz, int nb,
+                             int is_complex, const void* psi, double dV, double gx_dx, double gy_dy, double gz_dz,
+                             bool inner_only, void* ws, double** coef_out, cudaStream_t s) {
     const size_t N = (size_t)nx * ny * nz;
     const int ncol = is_complex ? 2 * nb : nb;
     const size_t part = (size_t)d.n_chunks * d.wmax * ncol * sizeof(double);
+    const size_t one = nl_workspace_bytes(d, ncol);
     double* partial = (double*)ws;
-    double* coef = (double*)((char*)ws + ((part + 255) / 256) * 256);
-    *coef_out = coef;
+    ProjTables tabs{};
+    for (int k = 0; k < ntab; ++k) {
+        coef_out[k] = (double*)((char*)ws + k * one + ((part + 255) / 256) * 256);
+        const int table = first_table + k;
+        const size_t toff = table < 0 ? 0 : (size_t)table * d.n_points * d.wmax;
+        if (dt == QSB_F64) tabs.t[k] = table < 0 ? d.pt_beta64 : d.pt_dbeta64 + toff;
+        else tabs.t[k] = table < 0 ? (const void*)d.pt_beta32 : (const void*)(d.pt_dbeta32 + toff);
+    }
     if (d.n_points == 0) return QSB_OK;
     if ((nb + 7) / 8 > 65535) return fail(QSB_ERR_INVALID, "nonlocal: too many bands");
+    const size_t stride = one / sizeof(double);
+    tabs.n = ntab;
+    // The tensor-core form where its rows are full: a complex bundle (the phases once per 32
+    // columns instead of once per 8: 48^3 x 24 bands, FP64, 45 -> 27 us) and the forces' four
+    // tables (0.73 against 1.07 ms at 96^3 x 128); one real table fills half of them and runs
+    // faster in the other (0.29 against 0.48 ms).  FP32 applies keep that one's order of sums.
+#define QSB_MMA(T, C) launch_proj_mma_w<T, C>(d, tabs, psi, N, gx_dx, gy_dy, gz_dz, partial, stride, ncol, s)
+#define QSB_VEC(T, C) launch_proj_w<T, C>(d, (const T*)tabs.t[0], nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s)
     if (dt == QSB_F64) {
-        if (is_complex) launch_proj_w<double, true>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
-        else launch_proj_w<double, false>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
+        if (is_complex) QSB_TRY((QSB_MMA(double, true)));
+        else if (ntab > 1) QSB_TRY((QSB_MMA(double, false)));
+        else QSB_TRY((QSB_VEC(double, false)));
     } else {
-        if (is_complex) launch_proj_w<float, true>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
-        else launch_proj_w<float, false>(d, table, nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s);
+        if (ntab > 1) QSB_TRY(is_complex ? (QSB_MMA(float, true)) : (QSB_MMA(float, false)));
+        else QSB_TRY(is_complex ? (QSB_VEC(float, true)) : (QSB_VEC(float, false)));
     }
-    QSB_CUDA_TRY(cudaGetLastError());
-    nl_finalize_kernel<<<d.n_atoms, 256, 0, s>>>(d.atom_chunk_begin, d.atom_chunk_end, d.atom_E, d.atom_width, d.wmax,
-                                                 partial, ncol, dV, inner_only ? 1 : 0, coef);
+#undef QSB_MMA
+#undef QSB_VEC
+    for (int k = 0; k < ntab; ++k)
+        nl_finalize_kernel<<<d.n_atoms, 256, 0, s>>>(d.atom_chunk_begin, d.atom_chunk_end, d.atom_E, d.atom_width,
+                                                     d.wmax, partial + k * stride, ncol, dV, inner_only ? 1 : 0,
+                                                     coef_out[k]);
     QSB_CUDA_TRY(cudaGetLastError());
     return QSB_OK;
 }
@@ -677,8 +1141,8 @@ qsb_status nl_project_table(qsb_dtype dt, const NLDevice& d, int table, int nx, 
 qsb_status nl_project(qsb_dtype dt, const NLDevice& d, int nx, int ny, int nz, int nb, int is_complex,
                       const void* psi, double dV, double gx_dx, double gy_dy, double gz_dz, bool inner_only, void* ws,
                       double** coef_out, cudaStream_t s) {
-    return nl_project_table(dt, d, -1, nx, ny, nz, nb, is_complex, psi, dV, gx_dx, gy_dy, gz_dz, inner_only, ws,
-                            coef_out, s);
+    return nl_project_tables(dt, d, -1, 1, nx, ny, nz, nb, is_complex, psi, dV, gx_dx, gy_dy, gz_dz, inner_only, ws,
+                             coef_out, s);
 }
 
 qsb_status nl_upload_gradients(NLDevice& d, const double* dbeta) {
@@ -726,9 +1190,11 @@ qsb_status nl_energy_force(qsb_dtype dt, const NLDevice& d, int nx, int ny, int 
     unsigned char* w = (unsigned char*)ws;
     double* coef[4] = {nullptr, nullptr, nullptr, nullptr};
     const int ntab = forces ? 4 : 1;
-    for (int t = 0; t < ntab; ++t)
-        QSB_TRY(nl_project_table(dt, d, t - 1, nx, ny, nz, nb, is_complex, psi, dV, gx_dx, gy_dy, gz_dz, true,
-                                 w + t * one, &coef[t], s));
+    // beta and its gradients share one gather of psi up to 4 projectors per atom (16 rows)
+    const int at_once = ntab == 4 && d.wmax <= 4 ? 4 : 1;
+    for (int t = 0; t < ntab; t += at_once)
+        QSB_TRY(nl_project_tables(dt, d, t - 1, at_once, nx, ny, nz, nb, is_complex, psi, dV, gx_dx, gy_dy, gz_dz,
+                                  true, w + t * one, &coef[t], s));
     double* out = (double*)(w + 4 * one);
     double* occ = out + (size_t)d.n_atoms * 4;
     QSB_CUDA_TRY(cudaMemcpyAsync(occ, occ_host, sizeof(double) * nb, cudaMemcpyHostToDevice, s));
@@ -754,21 +1220,18 @@ qsb_status nl_apply(qsb_dtype dt, const NLDevice& d, int N, int nb, int is_compl
     if (d.n_points == 0 || d.n_cov == 0) return QSB_OK;
     const int ncol = is_complex ? 2 * nb : nb;
     const dim3 grid((d.n_cov + APPLY_THREADS - 1) / APPLY_THREADS);
-    // v2 (coefficients staged in shared memory) while one slice of every atom's
-    // rows fits; QSB_NLAPPLY=v1 keeps the L1 form for A/B timing
-    static const bool force_v1 = [] {
-        const char* e = std::getenv("QSB_NLAPPLY");
-        return e && std::string(e) == "v1";
-    }();
-    const size_t smem2 = (size_t)d.n_atoms * d.wmax * APPLY_CW * sizeof(double);
-    const bool v2 = !force_v1 && smem2 <= 96 * 1024;
+    // pipelined form while two slices of the CTA's own atoms fit beside the ring (up to
+    // ~60 atoms x 4 projectors meeting in 256 points at two CTAs per SM); else per-point loads
 #define QSB_APPLY(T, C, W, B)                                                                                        \
     do {                                                                                                             \
-        if (v2) {                                                                                                    \
-            cudaFuncSetAttribute(nl_apply2_kernel<T, C, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2); \
-            nl_apply2_kernel<T, C, W><<<grid, APPLY_THREADS, smem2, s>>>(d.cov_grid, d.n_cov, d.grid_ptr, d.ent_atom, \
-                                                                         d.ent_xyz, B, d.wmax, d.n_atoms, coef, ncol, \
-                                                                         (T*)hpsi, (size_t)N, gx_dx, gy_dy, gz_dz);   \
+        const size_t smem = (size_t)ApplyCfg<T, C>::RING +                                                                \
+                            (size_t)2 * d.max_local * apply_row(d.wmax) * sizeof(double);                            \
+        if (smem <= 200 * 1024) {                                                                                    \
+            auto kern = d.wmax == W ? nl_apply_ring_kernel<T, C, W, true> : nl_apply_ring_kernel<T, C, W, false>;    \
+            QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));        \
+            kern<<<grid, APPLY_THREADS, smem, s>>>(d.cov_grid, d.n_cov, d.grid_ptr, d.ent_local, d.ent_xyz, B,       \
+                                                   d.wmax, d.cta_ptr, d.cta_atoms, d.max_local, coef, ncol,          \
+                                                   (T*)hpsi, (size_t)N, gx_dx, gy_dy, gz_dz);                        \
         } else {                                                                                                     \
             nl_apply_kernel<T, C, W><<<grid, APPLY_THREADS, 0, s>>>(d.cov_grid, d.n_cov, d.grid_ptr, d.ent_atom,      \
                                                                     d.ent_xyz, B, d.wmax, coef, ncol, (T*)hpsi,      \

@@ -138,6 +138,10 @@ struct NLDevice {
     int n_cov = 0;                 // grid points with at least one entry
     int* cov_grid = nullptr;       // [n_cov]
     int* ent_atom = nullptr;       // [n_points]
+    int* ent_local = nullptr;      // [n_points] place of the entry's atom in its run's list:
+    int* cta_ptr = nullptr;        //   run r (256 covered points) has the atoms
+    int* cta_atoms = nullptr;      //   cta_atoms[cta_ptr[r] .. cta_ptr[r + 1])
+    int max_local = 0;             // longest list
     int* ent_xyz = nullptr;        // [n_points][3]
     double* ent_beta64 = nullptr;  // [n_points][wmax]
     float* ent_beta32 = nullptr;
