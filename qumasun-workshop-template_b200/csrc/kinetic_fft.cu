@@ -22,7 +22,17 @@ namespace qsb {
 
 namespace {
 
-constexpr int FFT_CHUNK = 32;     // bands per batched transform
+constexpr int FFT_CHUNK = 32;     // most bands per batched transform
+// Spectra of one chunk of bands.  Each band's field is read and written by every
+// pass of the two transforms, the pack, the multiplier and the finish: chunks
+// whose spectra stay in the 126 MB L2 between the passes leave DRAM the psi
+// reads and H psi writes (at 32 bands, 226 MB of spectra at 96^3, every pass went
+// to DRAM).  A quarter of L2 beside the passes' psi and H psi.
+constexpr size_t FFT_L2_BYTES = 60u << 20;
+inline int fields_per_chunk(size_t field_bytes, int most) {
+    const size_t n = FFT_L2_BYTES / std::max<size_t>(1, field_bytes);
+    return (int)std::max<size_t>(1, std::min<size_t>((size_t)most, n));
+}
 constexpr int KT = 256;
 
 __device__ __forceinline__ double gfold(int m, int n, double c) { return c * (double)(2 * m > n ? m - n : m); }
@@ -50,22 +60,23 @@ __global__ void __launch_bounds__(KT) kmul_half_kernel(C* __restrict__ spec, siz
     }
 }
 
-// spectrum of complex bands: batch x nz x ny x nx
+// spectrum of complex bands: batch x nz x ny x nx (blockIdx.z: field, blockIdx.y: planes)
 template <typename C>
-__global__ void __launch_bounds__(KT) kmul_full_kernel(C* __restrict__ spec, size_t total, int nx, int ny, int nz,
-                                                       double cx, double cy, double cz, double kx0, double ky0,
-                                                       double kz0) {
-    for (size_t i = blockIdx.x * (size_t)KT + threadIdx.x; i < total; i += (size_t)gridDim.x * KT) {
-        const int kx = (int)(i % nx);
-        const size_t r = i / nx;
-        const int ky = (int)(r % ny);
-        const int kz = (int)((r / ny) % nz);
-        const double gx = gfold(kx, nx, cx) + kx0, gy = gfold(ky, ny, cy) + ky0, gz = gfold(kz, nz, cz) + kz0;
+__global__ void __launch_bounds__(KT) kmul_full_kernel(C* __restrict__ spec, int nx, int ny, int nz, double cx,
+                                                       double cy, double cz, double kx0, double ky0, double kz0) {
+    const unsigned nxy = (unsigned)nx * (unsigned)ny;
+    const unsigned i = blockIdx.x * KT + threadIdx.x;
+    if (i >= nxy) return;
+    const int ky = (int)(i / (unsigned)nx), kx = (int)(i - (unsigned)ky * (unsigned)nx);
+    const double gx = gfold(kx, nx, cx) + kx0, gy = gfold(ky, ny, cy) + ky0;
+    for (int kz = blockIdx.y; kz < nz; kz += gridDim.y) {
+        const double gz = gfold(kz, nz, cz) + kz0;
         const double m = 0.5 * (gx * gx + gy * gy + gz * gz);
-        C v = spec[i];
+        C* q = spec + ((size_t)blockIdx.z * nz + kz) * nxy + i;
+        C v = *q;
         v.x = (decltype(v.x))(v.x * m);
         v.y = (decltype(v.y))(v.y * m);
-        spec[i] = v;
+        *q = v;
     }
 }
 
@@ -78,64 +89,77 @@ __global__ void __launch_bounds__(KT) finish_real_kernel(T* __restrict__ hpsi, c
         hpsi[i] = (T)((double)hpsi[i] * inv_n) + V[i % N] * psi[i];
 }
 
-// complex SoA bands -> interleaved spectrum buffer
+// complex SoA bands -> interleaved spectrum buffer (blockIdx.y: band)
 template <typename T, typename C>
-__global__ void __launch_bounds__(KT) interleave_kernel(C* __restrict__ spec, const T* __restrict__ psi, size_t N,
-                                                        size_t total) {
-    for (size_t i = blockIdx.x * (size_t)KT + threadIdx.x; i < total; i += (size_t)gridDim.x * KT) {
-        const size_t b = i / N, p = i % N;
+__global__ void __launch_bounds__(KT) interleave_kernel(C* __restrict__ spec, const T* __restrict__ psi, size_t N) {
+    const T* re = psi + (size_t)2 * blockIdx.y * N;
+    C* out = spec + (size_t)blockIdx.y * N;
+    for (size_t p = blockIdx.x * (size_t)KT + threadIdx.x; p < N; p += (size_t)gridDim.x * KT) {
         C v;
-        v.x = psi[2 * b * N + p];
-        v.y = psi[(2 * b + 1) * N + p];
-        spec[i] = v;
+        v.x = re[p];
+        v.y = re[N + p];
+        out[p] = v;
     }
 }
 
-// complex bands: hpsi (SoA) = spectrum / N + V psi
+// complex bands: hpsi (SoA) = spectrum / N + V psi (blockIdx.y: band)
 template <typename T, typename C>
 __global__ void __launch_bounds__(KT) finish_cplx_kernel(T* __restrict__ hpsi, const C* __restrict__ spec,
                                                          const T* __restrict__ psi, const T* __restrict__ V,
-                                                         size_t N, size_t total, double inv_n) {
-    for (size_t i = blockIdx.x * (size_t)KT + threadIdx.x; i < total; i += (size_t)gridDim.x * KT) {
-        const size_t b = i / N, p = i % N;
-        const C v = spec[i];
+                                                         size_t N, double inv_n) {
+    const size_t o = (size_t)2 * blockIdx.y * N;
+    const C* in = spec + (size_t)blockIdx.y * N;
+    for (size_t p = blockIdx.x * (size_t)KT + threadIdx.x; p < N; p += (size_t)gridDim.x * KT) {
+        const C v = in[p];
         const T vp = V[p];
-        const size_t re = 2 * b * N + p, im = re + N;
-        hpsi[re] = (T)((double)v.x * inv_n) + vp * psi[re];
-        hpsi[im] = (T)((double)v.y * inv_n) + vp * psi[im];
+        hpsi[o + p] = (T)((double)v.x * inv_n) + vp * psi[o + p];
+        hpsi[o + N + p] = (T)((double)v.y * inv_n) + vp * psi[o + N + p];
     }
 }
 
-// real bands, two to a complex field: spec[p] = psi[2p] + i psi[2p+1] (zero
+// real bands, two to a complex field (blockIdx.y): spec[p] = psi[2p] + i psi[2p+1] (zero
 // imaginary part for an odd last band).  The multiplier is real and even at
 // k = 0, so the kinetic operator is real and acts on the two bands
 // independently: T(a + ib) = Ta + iTb.
 template <typename T, typename C>
 __global__ void __launch_bounds__(KT) pack_pairs_kernel(C* __restrict__ spec, const T* __restrict__ psi, size_t N,
-                                                        int bands, size_t total) {
-    for (size_t i = blockIdx.x * (size_t)KT + threadIdx.x; i < total; i += (size_t)gridDim.x * KT) {
-        const size_t pr = i / N, p = i - pr * N;
-        const size_t b0 = 2 * pr;
+                                                        int bands) {
+    const size_t b0 = (size_t)2 * blockIdx.y;
+    const bool two = (int)b0 + 1 < bands;
+    const T* in = psi + b0 * N;
+    C* out = spec + (size_t)blockIdx.y * N;
+    for (size_t p = blockIdx.x * (size_t)KT + threadIdx.x; p < N; p += (size_t)gridDim.x * KT) {
         C v;
-        v.x = psi[b0 * N + p];
-        v.y = (int)b0 + 1 < bands ? psi[(b0 + 1) * N + p] : (T)0;
-        spec[i] = v;
+        v.x = in[p];
+        v.y = two ? in[N + p] : (T)0;
+        out[p] = v;
     }
 }
 
-// hpsi[2p] = Re spec[p] / N + V psi[2p], hpsi[2p+1] = Im spec[p] / N + V psi[2p+1]
+// hpsi[2p] = Re spec[p] / N + V psi[2p], hpsi[2p+1] = Im spec[p] / N + V psi[2p+1] (blockIdx.y: p)
 template <typename T, typename C>
 __global__ void __launch_bounds__(KT) finish_pairs_kernel(T* __restrict__ hpsi, const C* __restrict__ spec,
                                                           const T* __restrict__ psi, const T* __restrict__ V,
-                                                          size_t N, int bands, size_t total, double inv_n) {
-    for (size_t i = blockIdx.x * (size_t)KT + threadIdx.x; i < total; i += (size_t)gridDim.x * KT) {
-        const size_t pr = i / N, p = i - pr * N;
-        const size_t b0 = 2 * pr;
-        const C v = spec[i];
+                                                          size_t N, int bands, double inv_n) {
+    const size_t b0 = (size_t)2 * blockIdx.y;
+    const bool two = (int)b0 + 1 < bands;
+    const T* x = psi + b0 * N;
+    T* y = hpsi + b0 * N;
+    const C* in = spec + (size_t)blockIdx.y * N;
+    for (size_t p = blockIdx.x * (size_t)KT + threadIdx.x; p < N; p += (size_t)gridDim.x * KT) {
+        const C v = in[p];
         const T vp = V[p];
-        hpsi[b0 * N + p] = (T)((double)v.x * inv_n) + vp * psi[b0 * N + p];
-        if ((int)b0 + 1 < bands) hpsi[(b0 + 1) * N + p] = (T)((double)v.y * inv_n) + vp * psi[(b0 + 1) * N + p];
+        y[p] = (T)((double)v.x * inv_n) + vp * x[p];
+        if (two) y[N + p] = (T)((double)v.y * inv_n) + vp * x[N + p];
     }
+}
+
+// N points of `fields` fields
+inline dim3 grid_fields(size_t N, int fields) {
+    return dim3((unsigned)std::max<size_t>(1, std::min<size_t>((N + KT - 1) / KT, 148 * 16)), (unsigned)fields);
+}
+inline dim3 grid_planes(int nx, int ny, int nz, int fields) {
+    return dim3((unsigned)(((size_t)nx * ny + KT - 1) / KT), (unsigned)std::min(nz, 65535), (unsigned)fields);
 }
 
 unsigned grid_for(size_t total) {
@@ -185,8 +209,8 @@ qsb_status apply_t(qsb_ham* h, qsb_dtype dtype, int cplx, int nb, const T* psi, 
         // real bands in pairs through the complex transforms: cuFFT's complex
         // passes run at ~4.8 TB/s where its x-direction R2C / C2R kernels run
         // at ~1.65 TB/s on these grids
-        const int chunk = std::min(nb, FFT_CHUNK);
-        const int pmax = (chunk + 1) / 2;
+        const int pmax = fields_per_chunk(N * sizeof(C), std::min((nb + 1) / 2, FFT_CHUNK / 2));
+        const int chunk = 2 * pmax;
         const size_t need = (size_t)pmax * N * sizeof(C);
         if (h->fft_buf_bytes < need) {
             if (h->fft_buf) QSB_CUDA_TRY(cudaFree(h->fft_buf));
@@ -208,23 +232,22 @@ qsb_status apply_t(qsb_ham* h, qsb_dtype dtype, int cplx, int nb, const T* psi, 
             QSB_FFT_TRY(cufftSetStream((cufftHandle)p->forward, s));
             const T* x = psi + (size_t)b0 * N;
             T* y = hpsi + (size_t)b0 * N;
-            const size_t npts = (size_t)pairs * N;
-            pack_pairs_kernel<T, C><<<grid_for(npts), KT, 0, s>>>(spec, x, N, bc, npts);
+            pack_pairs_kernel<T, C><<<grid_fields(N, pairs), KT, 0, s>>>(spec, x, N, bc);
             QSB_CUDA_TRY(cudaGetLastError());
             if constexpr (sizeof(T) == 8) {
                 QSB_FFT_TRY(cufftExecZ2Z((cufftHandle)p->forward, spec, spec, CUFFT_FORWARD));
             } else {
                 QSB_FFT_TRY(cufftExecC2C((cufftHandle)p->forward, spec, spec, CUFFT_FORWARD));
             }
-            kmul_full_kernel<C><<<grid_for(npts), KT, 0, s>>>(spec, npts, h->nx, h->ny, h->nz, cx, cy, cz, 0.0, 0.0,
-                                                               0.0);
+            kmul_full_kernel<C><<<grid_planes(h->nx, h->ny, h->nz, pairs), KT, 0, s>>>(spec, h->nx, h->ny, h->nz, cx,
+                                                                                      cy, cz, 0.0, 0.0, 0.0);
             QSB_CUDA_TRY(cudaGetLastError());
             if constexpr (sizeof(T) == 8) {
                 QSB_FFT_TRY(cufftExecZ2Z((cufftHandle)p->backward, spec, spec, CUFFT_INVERSE));
             } else {
                 QSB_FFT_TRY(cufftExecC2C((cufftHandle)p->backward, spec, spec, CUFFT_INVERSE));
             }
-            finish_pairs_kernel<T, C><<<grid_for(npts), KT, 0, s>>>(y, spec, x, V, N, bc, npts, inv_n);
+            finish_pairs_kernel<T, C><<<grid_fields(N, pairs), KT, 0, s>>>(y, spec, x, V, N, bc, inv_n);
             QSB_CUDA_TRY(cudaGetLastError());
             *launches += 3;
         }
@@ -232,7 +255,7 @@ qsb_status apply_t(qsb_ham* h, qsb_dtype dtype, int cplx, int nb, const T* psi, 
     }
     const int nxh = h->nx / 2 + 1;
     const size_t spec_per_band = cplx ? N : (size_t)h->nz * h->ny * nxh;
-    const int chunk = std::min(nb, FFT_CHUNK);
+    const int chunk = fields_per_chunk(spec_per_band * sizeof(C), std::min(nb, FFT_CHUNK));
     const size_t need = (size_t)chunk * spec_per_band * sizeof(C);
     if (h->fft_buf_bytes < need) {
         if (h->fft_buf) QSB_CUDA_TRY(cudaFree(h->fft_buf));
@@ -274,22 +297,22 @@ qsb_status apply_t(qsb_ham* h, qsb_dtype dtype, int cplx, int nb, const T* psi, 
             QSB_CUDA_TRY(cudaGetLastError());
             *launches += 2;
         } else {
-            interleave_kernel<T, C><<<grid_for(npts), KT, 0, s>>>(spec, x, N, npts);
+            interleave_kernel<T, C><<<grid_fields(N, bc), KT, 0, s>>>(spec, x, N);
             QSB_CUDA_TRY(cudaGetLastError());
             if constexpr (sizeof(T) == 8) {
                 QSB_FFT_TRY(cufftExecZ2Z((cufftHandle)p->forward, spec, spec, CUFFT_FORWARD));
             } else {
                 QSB_FFT_TRY(cufftExecC2C((cufftHandle)p->forward, spec, spec, CUFFT_FORWARD));
             }
-            kmul_full_kernel<C><<<grid_for(nspec), KT, 0, s>>>(spec, nspec, h->nx, h->ny, h->nz, cx, cy, cz, gx, gy,
-                                                                gz);
+            kmul_full_kernel<C><<<grid_planes(h->nx, h->ny, h->nz, bc), KT, 0, s>>>(spec, h->nx, h->ny, h->nz, cx, cy,
+                                                                                   cz, gx, gy, gz);
             QSB_CUDA_TRY(cudaGetLastError());
             if constexpr (sizeof(T) == 8) {
                 QSB_FFT_TRY(cufftExecZ2Z((cufftHandle)p->backward, spec, spec, CUFFT_INVERSE));
             } else {
                 QSB_FFT_TRY(cufftExecC2C((cufftHandle)p->backward, spec, spec, CUFFT_INVERSE));
             }
-            finish_cplx_kernel<T, C><<<grid_for(npts), KT, 0, s>>>(y, spec, x, V, N, npts, inv_n);
+            finish_cplx_kernel<T, C><<<grid_fields(N, bc), KT, 0, s>>>(y, spec, x, V, N, inv_n);
             QSB_CUDA_TRY(cudaGetLastError());
             *launches += 3;
         }
