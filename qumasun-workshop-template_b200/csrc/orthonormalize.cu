@@ -100,7 +100,8 @@ extern "C" qsb_status qsb_orthonormalize(int64_t N, int nb, int is_complex, doub
         ORTH_SOLVER(cusolverDnZpotrf_bufferSize(h.sol, CUBLAS_FILL_MODE_UPPER, n, nullptr, n, &lwork));
     else
         ORTH_SOLVER(cusolverDnDpotrf_bufferSize(h.sol, CUBLAS_FILL_MODE_UPPER, n, nullptr, n, &lwork));
-    const size_t w_doubles = (size_t)lwork * (is_complex ? 2 : 1) + 2 + n;
+    // an even number of doubles, so that the interleaved bundle behind them is 16-byte aligned
+    const size_t w_doubles = ((size_t)lwork * (is_complex ? 2 : 1) + 2 + n + 1) & ~(size_t)1;
     const size_t z_doubles = is_complex ? (size_t)2 * N * n : 0;
     QSB_CUDA_TRY(cudaMalloc(&h.mem, sizeof(double) * (t_doubles + g_doubles + w_doubles + z_doubles) + 64));
     double* T = (double*)h.mem;
