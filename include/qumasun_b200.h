@@ -141,7 +141,8 @@ QSB_API qsb_status qsb_ham_apply(qsb_ham* ham, qsb_dtype dtype, int is_complex, 
  *      times |G + k|^2 / 2 with the Nyquist index of an even grid taken as
  *      +n/2 (OperateKineticInKspace_bundle :96-123), inverse FFT, times 1/N,
  *      + V psi, + the nonlocal part.  Batched cuFFT plans and a spectrum
- *      buffer for 32 bands are made on first use and kept in the context.
+ *      buffer for a chunk of bands (up to 32, as many as stay in L2) are made
+ *      on first use and kept in the context.
  *      FP64 and FP32 (the mixed solver's operator). */
 QSB_API qsb_status qsb_ham_set_kinetic(qsb_ham* ham, int algorithm);
 
@@ -162,12 +163,13 @@ QSB_API qsb_status qsb_ham_apply_host(qsb_ham* ham, qsb_dtype dtype, int is_comp
 
 /* H psi of n_sys independent systems at once (real bands, Gamma point, FD8
  * kinetic): hpsi[i] = H_i psi[i] for nb[i] bands of system i (each its own
- * qsb_ham: grid, spacing, potential, projectors).  The FD8 + V part of all
- * systems runs in ONE persistent launch over a work list of (system, tile of
- * 32 x 16 points (FP32: 32 x 32), 32-plane z chunk, band) items, largest
- * systems first, each item the tile work of the register-prefetch stencil
- * (results equal the per-system FP32 stencil's bit for bit); each system's
- * nonlocal projection and expansion keep their own launches.  The reference
+ * qsb_ham: grid, spacing, potential, projectors).  The FD8 + V part of the
+ * systems that do not fill the GPU on their own runs in ONE persistent launch
+ * over a work list of (system, tile of 32 x 16 points (FP32: 32 x 32), 32-plane
+ * z chunk, band) items, largest systems first, each item the tile work of the
+ * register-prefetch stencil (FP32 results equal the per-system stencil's bit for
+ * bit); larger systems and each system's nonlocal projection and expansion keep
+ * their own launches.  The reference
  * applies H system by system (mHamiltonianMatrix_ddm, source/qumasun_base1.matrix.h:263-291);
  * for many small, uneven cells a launch per system leaves most SMs idle.
  * Results equal qsb_ham_apply's to rounding (a different stencil kernel).

@@ -1,6 +1,6 @@
 // qsb_ham_apply_batch: H psi for many independent systems (different grids,
-// band counts and projector sets) with the FD8 + V part of all of them in ONE
-// persistent launch.
+// band counts and projector sets) with the FD8 + V part of all those that do not
+// fill the GPU on their own in ONE persistent launch.
 //
 // The reference solves its systems one after another, each call a launch per
 // operator piece; for a set of small, uneven cells (32^3 .. 64^3 grids, 8 .. 64
@@ -123,15 +123,27 @@ qsb_status apply_batched(qsb_dtype dtype, int n_sys, qsb_ham* const* hams, const
                                 0.0, false, h->ws, &coef[i], s));
         launches += 2;
     }
-    // 2) V psi - 1/2 FD8 psi of all systems in one persistent launch
-    std::vector<qsb::BatchSysDesc> d(n_sys);
+    // 2) V psi - 1/2 FD8 psi: a system whose own tiles fill the GPU by the TMA-fed stencil, the
+    //    others together in one persistent launch (of the register-prefetch kernel's tile work,
+    //    bound by instruction issue: 12 cells of 32^3 to 64^3, 8 to 64 bands, 0.49 ms all
+    //    together, 0.42 with the nine large ones apart)
+    std::vector<qsb::BatchSysDesc> d;
     for (int i = 0; i < n_sys; ++i) {
         const qsb_ham* h = hams[i];
-        d[i] = qsb::BatchSysDesc{psi[i], hpsi[i], dtype == QSB_F64 ? (const void*)h->V64 : (const void*)h->V32,
-                                 h->nx, h->ny, h->nz, nb[i], qsb::make_fd8_coef(-0.5, h->dx, h->dy, h->dz, 0, 0, 0)};
+        const void* V = dtype == QSB_F64 ? (const void*)h->V64 : (const void*)h->V32;
+        const qsb::FD8Coef c = qsb::make_fd8_coef(-0.5, h->dx, h->dy, h->dz, 0, 0, 0);
+        if (nb[i] > 0 && qsb::stencil_fills_gpu(h->nx, h->ny, h->nz, nb[i])) {
+            qsb::StencilLaunch L{h->nx, h->ny, h->nz, nb[i], 0, 1, psi[i], hpsi[i], V};
+            QSB_TRY(qsb::launch_stencil(dtype, L, c, s));
+            ++launches;
+        } else {
+            d.push_back(qsb::BatchSysDesc{psi[i], hpsi[i], V, h->nx, h->ny, h->nz, nb[i], c});
+        }
     }
-    QSB_TRY(qsb::launch_stencil_batch(dtype, n_sys, d.data(), s));
-    ++launches;
+    if (!d.empty()) {
+        QSB_TRY(qsb::launch_stencil_batch(dtype, (int)d.size(), d.data(), s));
+        ++launches;
+    }
     // 3) + the nonlocal expansion of every system
     for (int i = 0; i < n_sys; ++i) {
         if (!coef[i]) continue;

@@ -100,6 +100,9 @@ struct BatchSysDesc {
     FD8Coef coef;
 };
 qsb_status launch_stencil_batch(qsb_dtype dt, int n, const BatchSysDesc* d, cudaStream_t s);
+// Whether the TMA-fed stencils cover this real bundle's grid and its tiles x bands x 16-plane
+// chunks are enough CTAs for every SM.
+bool stencil_fills_gpu(int nx, int ny, int nz, int nb);
 // Autotuner state (stencil.cu): whether qsb_set_autotune is on, and a line for
 // the decision log qsb_autotune_report returns.
 bool autotune_enabled();

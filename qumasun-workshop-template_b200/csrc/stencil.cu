@@ -65,6 +65,14 @@ __device__ __forceinline__ int wrapi(int v, int n) {
     return m < 0 ? m + n : m;
 }
 
+// v >= 0 wrapped into [0, n): one compare where v < 2 n (a plane or two past the end), the
+// remainder only on grids thinner than the stencil.  The register kernel is bound by
+// instruction issue, and two remainders per plane were a fifth of its instructions.
+__device__ __forceinline__ int wrap_up(int v, int n) {
+    v = v >= n ? v - n : v;
+    return v < n ? v : v % n;
+}
+
 // One CTA: a TX x TY tile (TY = BY*RY) of one band (both SoA planes for
 // complex), marching z over [z0, z1).  Thread (tx, ty) owns the RY
 // consecutive grid rows y0 + ty*RY + i at x0 + tx and keeps their z columns
@@ -185,7 +193,7 @@ __device__ __forceinline__ void fd8_tile(const T* __restrict__ in, T* __restrict
             if (z < z1) {
                 const int buf = (z - z0) & 1;
                 T* sb = &sm[buf][0][0][0];
-                const size_t zo2 = nxy * (size_t)wrapi(z + 2, nz);
+                const size_t zo2 = nxy * (size_t)wrap_up(z + 2, nz);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     if (xh_ok) sb[c * SH * SW + xh_s] = hx[p % 3][c];
@@ -205,7 +213,7 @@ __device__ __forceinline__ void fd8_tile(const T* __restrict__ in, T* __restrict
                         ep[(p + 2) % 3][0][i] = ok ? __ldg(V + o2) : T(0);
                     }
                 }
-                const size_t zo4 = nxy * (size_t)wrapi(z + HW, nz);
+                const size_t zo4 = nxy * (size_t)wrap_up(z + HW, nz);
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -2018,6 +2026,12 @@ qsb_status stencil_batch_t(int n, const BatchSysDesc* d, cudaStream_t s) {
 
 qsb_status launch_stencil_batch(qsb_dtype dt, int n, const BatchSysDesc* d, cudaStream_t s) {
     return dt == QSB_F64 ? stencil_batch_t<double>(n, d, s) : stencil_batch_t<float>(n, d, s);
+}
+
+bool stencil_fills_gpu(int nx, int ny, int nz, int nb) {
+    const long long tiles = (long long)((nx + ZTX - 1) / ZTX) * ((ny + 31) / 32);
+    return nx % 4 == 0 && ws_dim_ok(nx, ZTX) && ws_dim_ok(ny, 32) && nz >= HW &&
+           tiles * nb * std::max(1, nz / 16) >= sm_count();
 }
 
 bool autotune_enabled() { return tune_state().on; }
