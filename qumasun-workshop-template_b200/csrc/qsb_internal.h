@@ -184,6 +184,13 @@ qsb_status nl_project(qsb_dtype dt, const NLDevice& d, int nx, int ny, int nz, i
 qsb_status nl_apply(qsb_dtype dt, const NLDevice& d, int N, int nb, int is_complex, void* hpsi,
                     const double* coef, double gx_dx, double gy_dy, double gz_dz, cudaStream_t s);
 
+// Lowest n eigenpairs of an m x m Hermitian (cplx: interleaved complex) or
+// symmetric definite pencil in one launch (pencil_small.cu): eigenvalues to W,
+// B-orthonormal vectors to the first n columns of Sa (ld m); Sb is overwritten.
+// *info (device): 0, m + k (order-k minor of Sb not positive), -1 (not resolved).
+bool pencil_small_fits(int m, int n, bool cplx);
+qsb_status pencil_small(int m, int n, bool cplx, double* Sa, double* Sb, double* W, int* info, cudaStream_t s);
+
 // Split-BF16x3 tensor-core Gram products (gram_tc.cu).
 //
 // A tall operand is a set of columns of N grid values (fp32 or fp64, one
