@@ -33,15 +33,25 @@ namespace qsb {
 namespace {
 
 constexpr int RED_THREADS = 256;
-constexpr int RED_CHUNK = 1 << 16;   // doubles per reduction block
+constexpr int RED_CHUNK = 1 << 16;   // elements per reduction block (mixed precision)
+
+// Elements per reduction block of a context: the FP64 solvers cut a band into up to 32 pieces of
+// 4096 or more, so that a few bands of a small grid fill the GPU (16 bands of 32^3: 16 blocks
+// of 65536, 14 us a pass, against 128 of 4096, 3 us).  The mixed solver keeps the longer
+// ones: its results depend on the order of these sums.
+inline int red_chunk_of(size_t L, bool mixed) {
+    if (mixed) return RED_CHUNK;
+    const size_t piece = ((L + 31) / 32 + 1023) / 1024 * 1024;
+    return (int)std::min<size_t>(RED_CHUNK, std::max<size_t>(4096, piece));
+}
 
 // partial[s * nch + ch] = sum over chunk ch of segment s of a[i]*b[i]
 // (fp64 or fp32 bundles, fp64 sums)
 template <typename T>
-__global__ void seg_dot_partial(const T* __restrict__ a, const T* __restrict__ b, size_t L, int nch,
+__global__ void seg_dot_partial(const T* __restrict__ a, const T* __restrict__ b, size_t L, int chunk, int nch,
                                 double* __restrict__ partial) {
     const int s = blockIdx.y, ch = blockIdx.x;
-    const size_t i0 = (size_t)ch * RED_CHUNK, i1 = min(L, i0 + RED_CHUNK);
+    const size_t i0 = (size_t)ch * chunk, i1 = min(L, i0 + chunk);
     const T* A = a + (size_t)s * L;
     const T* B = b + (size_t)s * L;
     double acc = 0.0;
@@ -60,9 +70,10 @@ __global__ void seg_dot_partial(const T* __restrict__ a, const T* __restrict__ b
 // r = ax - eps[s]*x; partial sums of r^2 (if partial != nullptr)
 template <typename T>
 __global__ void seg_residual_partial(T* __restrict__ r, const T* __restrict__ ax, const T* __restrict__ x,
-                                     const double* __restrict__ eps, size_t L, int nch, double* __restrict__ partial) {
+                                     const double* __restrict__ eps, size_t L, int chunk, int nch,
+                                     double* __restrict__ partial) {
     const int s = blockIdx.y, ch = blockIdx.x;
-    const size_t i0 = (size_t)ch * RED_CHUNK, i1 = min(L, i0 + RED_CHUNK);
+    const size_t i0 = (size_t)ch * chunk, i1 = min(L, i0 + chunk);
     const size_t off = (size_t)s * L;
     const double e = eps[s];
     double acc = 0.0;
@@ -90,6 +101,48 @@ __global__ void seg_finalize(const double* __restrict__ partial, int nseg, int n
     double t = 0.0;
     for (int c = 0; c < nch; ++c) t += partial[(size_t)s * nch + c];
     out[s] = t * scale;
+}
+
+// sums as seg_finalize, and their inverse square roots
+__global__ void seg_finalize_rsqrt(const double* __restrict__ partial, int nseg, int nch, double scale,
+                                   double* __restrict__ out, double* __restrict__ inv) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nseg) return;
+    double t = 0.0;
+    for (int c = 0; c < nch; ++c) t += partial[(size_t)s * nch + c];
+    out[s] = t * scale;
+    inv[s] = 1.0 / sqrt(t * scale);
+}
+
+// out[s] = in[s] * scale[s] and, with partial, partial sums of out[s] * y[s] in
+// seg_dot_partial's order: the copy, the scaling and the inner product of a
+// rotated bundle in one pass (three took 9 bytes moved per byte of it, this 3).
+template <bool DOT>
+__global__ void seg_scale_to(const double* __restrict__ in, double* __restrict__ out, const double* __restrict__ scale,
+                             const double* __restrict__ y, size_t L, int chunk, int nch,
+                             double* __restrict__ partial) {
+    const int s = blockIdx.y, ch = blockIdx.x;
+    const size_t i0 = (size_t)ch * chunk, i1 = min(L, i0 + chunk);
+    const size_t off = (size_t)s * L;
+    const double c = scale[s];
+    double acc = 0.0;
+#pragma unroll 4
+    for (size_t i = i0 + threadIdx.x; i < i1; i += RED_THREADS) {
+        const double v = in[off + i] * c;
+        out[off + i] = v;
+        if (DOT) acc += v * y[off + i];
+    }
+    if constexpr (DOT) {
+        __shared__ double red[RED_THREADS / 32];
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+            for (int w = 0; w < RED_THREADS / 32; ++w) t += red[w];
+            partial[(size_t)s * nch + ch] = t;
+        }
+    }
 }
 
 // x[s] *= scale[s]  (or a single scalar when scale == nullptr)
@@ -254,7 +307,8 @@ struct qsb_eigensolver {
     double* rc = nullptr;            // rotation coefficient views, 6 x (2n x n)
     double* vec = nullptr;           // small per-band vectors (eps, norms, scales): 8 x nmax
     double* partial = nullptr;       // reduction partials: nmax x nch
-    int nch = 0;
+    double* gsmall = nullptr;        // tiles of the small real pencil (gram_small), few bands only
+    int nch = 0, chunk = 0;          // pieces of a band in the reductions, elements per piece
     void* swork = nullptr;
     int slwork = 0;
     int* info = nullptr;
@@ -334,9 +388,35 @@ qsb_status seg_convert_by(qsb_eigensolver* es, int nseg, const Ti* in, To* out, 
 template <typename T>
 qsb_status seg_dot(qsb_eigensolver* es, int nseg, const T* a, const T* b, double scale, double* out, cudaStream_t s) {
     if (nseg <= 0) return QSB_OK;
-    const int nch = (int)((es->L + RED_CHUNK - 1) / RED_CHUNK);
-    seg_dot_partial<<<dim3(nch, nseg), RED_THREADS, 0, s>>>(a, b, es->L, nch, es->partial);
+    const int nch = es->nch;
+    seg_dot_partial<<<dim3(nch, nseg), RED_THREADS, 0, s>>>(a, b, es->L, es->chunk, nch, es->partial);
     seg_finalize<<<(nseg + 127) / 128, 128, 0, s>>>(es->partial, nseg, nch, scale, out);
+    QSB_CUDA_TRY(cudaGetLastError());
+    return QSB_OK;
+}
+
+// norms[s] = scale * sum(a_s^2), inv[s] = 1 / sqrt(norms[s]) (device vectors)
+qsb_status seg_norms(qsb_eigensolver* es, int nseg, const double* a, double scale, double* norms, double* inv,
+                     cudaStream_t s) {
+    if (nseg <= 0) return QSB_OK;
+    const int nch = es->nch;
+    seg_dot_partial<<<dim3(nch, nseg), RED_THREADS, 0, s>>>(a, a, es->L, es->chunk, nch, es->partial);
+    seg_finalize_rsqrt<<<(nseg + 127) / 128, 128, 0, s>>>(es->partial, nseg, nch, scale, norms, inv);
+    QSB_CUDA_TRY(cudaGetLastError());
+    return QSB_OK;
+}
+
+// out_s = in_s * f[s]; with y: dot[s] = scale * sum(out_s * y_s)
+qsb_status seg_scaled_copy(qsb_eigensolver* es, int nseg, const double* in, double* out, const double* f,
+                           const double* y, double scale, double* dot, cudaStream_t s) {
+    if (nseg <= 0) return QSB_OK;
+    const int nch = es->nch;
+    if (y) {
+        seg_scale_to<true><<<dim3(nch, nseg), RED_THREADS, 0, s>>>(in, out, f, y, es->L, es->chunk, nch, es->partial);
+        seg_finalize<<<(nseg + 127) / 128, 128, 0, s>>>(es->partial, nseg, nch, scale, dot);
+    } else {
+        seg_scale_to<false><<<dim3(nch, nseg), RED_THREADS, 0, s>>>(in, out, f, nullptr, es->L, es->chunk, nch, nullptr);
+    }
     QSB_CUDA_TRY(cudaGetLastError());
     return QSB_OK;
 }
@@ -345,8 +425,8 @@ template <typename T>
 qsb_status seg_residual(qsb_eigensolver* es, int nseg, T* r, const T* ax, const T* x, const double* eps,
                         double* norms, double scale, cudaStream_t s) {
     if (nseg <= 0) return QSB_OK;
-    const int nch = (int)((es->L + RED_CHUNK - 1) / RED_CHUNK);
-    seg_residual_partial<<<dim3(nch, nseg), RED_THREADS, 0, s>>>(r, ax, x, eps, es->L, nch,
+    const int nch = es->nch;
+    seg_residual_partial<<<dim3(nch, nseg), RED_THREADS, 0, s>>>(r, ax, x, eps, es->L, es->chunk, nch,
                                                                  norms ? es->partial : nullptr);
     if (norms) seg_finalize<<<(nseg + 127) / 128, 128, 0, s>>>(es->partial, nseg, nch, scale, norms);
     QSB_CUDA_TRY(cudaGetLastError());
@@ -1231,6 +1311,9 @@ qsb_status qsb_eigensolver_create_ex(qsb_eigensolver** out, int64_t N, int n, in
         cudaSuccess)
         return cleanup(fail(QSB_ERR_NOMEM, "eigensolver: pencil workspace allocation"));
     if (!es->mixed) es->drop_tol = 1e-12;
+    if (!es->mixed && !is_complex && gram_small_doubles(n) > 0 &&
+        cudaMalloc((void**)&es->gsmall, gram_small_doubles(n) * sizeof(double)) != cudaSuccess)
+        return cleanup(fail(QSB_ERR_NOMEM, "eigensolver: pencil tile allocation"));
     if (!es->mixed && is_complex) {
         const size_t mx = (size_t)3 * n;
         if (cudaMalloc((void**)&es->nxt, sizeof(double2) * (2 * mx * mx + (size_t)6 * n * n + 2 * mx * n)) !=
@@ -1240,7 +1323,8 @@ qsb_status qsb_eigensolver_create_ex(qsb_eigensolver** out, int64_t N, int n, in
     const int m = 3 * n;
     const size_t cm = (size_t)m * m * (is_complex ? 2 : 1);
     const size_t tsz = (size_t)(2 * n) * (2 * n);
-    es->nch = (int)((es->L + RED_CHUNK - 1) / RED_CHUNK);
+    es->chunk = red_chunk_of(es->L, es->mixed != 0);
+    es->nch = (int)((es->L + es->chunk - 1) / es->chunk);
     const size_t small = tsz + 2 * cm + m + (size_t)6 * 2 * n * n + 8 * (size_t)n + (size_t)n * es->nch;
     double* base = nullptr;
     if (cudaMalloc((void**)&base, small * sizeof(double)) != cudaSuccess)
@@ -1266,7 +1350,7 @@ qsb_status qsb_eigensolver_destroy(qsb_eigensolver* es) {
     float* b32[7] = {es->X32, es->R32, es->P32, es->AX32, es->AR32, es->AP32, es->TMP32};
     for (float* p : b32)
         if (p) cudaFree(p);
-    void* mw[9] = {es->su, es->sau, es->gpart, es->T2, es->rc32, es->svq, es->rotw, es->rotc, es->nxt};
+    void* mw[10] = {es->su, es->sau, es->gpart, es->T2, es->rc32, es->svq, es->rotw, es->rotc, es->nxt, es->gsmall};
     for (void* p : mw)
         if (p) cudaFree(p);
     if (es->T) cudaFree(es->T);
@@ -1496,6 +1580,8 @@ qsb_status qsb_lobpcg_z(qsb_eigensolver* es, double dVol, int n, int iter_max, d
             // ||X'||^2 (:2570) and the rollback test (:2611-2666)
             QSB_TRY(seg_dot(es, N_, es->TMP, es->TMP, 1.0, nrm_d, s));
             QSB_CUDA_TRY(cudaMemcpyAsync(nx.data(), nrm_d, sizeof(double) * N_, cudaMemcpyDeviceToHost, s));
+            std::vector<double> w(N_);                       // the Ritz values, in the same wait
+            QSB_CUDA_TRY(cudaMemcpyAsync(w.data(), es->W, sizeof(double) * N_, cudaMemcpyDeviceToHost, s));
             QSB_CUDA_TRY(cudaStreamSynchronize(s));
             double maxdiff = 0.0;
             for (int k = 0; k < N_; ++k) {
@@ -1517,9 +1603,6 @@ qsb_status qsb_lobpcg_z(qsb_eigensolver* es, double dVol, int n, int iter_max, d
                 break;
             }
             QSB_CUDA_TRY(cudaMemcpyAsync(band(X, head), es->TMP, sizeof(double) * L * N_, cudaMemcpyDeviceToDevice, s));
-            std::vector<double> w(N_);
-            QSB_CUDA_TRY(cudaMemcpyAsync(w.data(), es->W, sizeof(double) * N_, cudaMemcpyDeviceToHost, s));
-            QSB_CUDA_TRY(cudaStreamSynchronize(s));
             for (int k = 0; k < N_; ++k) eps[head + k] = w[k];
             const bool final_step = (iter + 1 == iter_max);
             if (!final_step) {
@@ -1578,8 +1661,13 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     const size_t L = es->L;
     double* eps_d = es->vec;
     double* nrm_d = es->vec + n;
-    double* scl_d = es->vec + 2 * n;
-    std::vector<double> v(n), scl(n);
+    // eps, |r|^2, |x|^2, |p|^2 next to each other (one copy to the host per iteration), then
+    // the factors of x and p, and the scale of the initial normalisations
+    double* xn_d = es->vec + 2 * n;
+    double* pn_d = es->vec + 3 * n;
+    double* sx_d = es->vec + 4 * n;
+    double* sp_d = es->vec + 5 * n;
+    std::vector<double> v(n);
 
     auto host_vec = [&](const double* d, std::vector<double>& h) -> qsb_status {
         QSB_CUDA_TRY(cudaMemcpyAsync(h.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
@@ -1588,18 +1676,15 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
             if (!std::isfinite(h[k])) return fail(QSB_ERR_NUMERIC, "lobpcg_d: non-finite value");
         return QSB_OK;
     };
-    auto normalize = [&](double* B, std::vector<double>* norms_out) -> qsb_status {
-        // Normalize (source/vecmath.h:128-134): x /= sqrt(|x|^2 dV), returns |x|^2 dV
-        QSB_TRY(seg_dot(es, n, B, B, dVol, nrm_d, s));
-        QSB_TRY(host_vec(nrm_d, v));
-        for (int k = 0; k < n; ++k) scl[k] = 1.0 / std::sqrt(v[k]);
-        if (norms_out) *norms_out = v;
-        QSB_CUDA_TRY(cudaMemcpyAsync(scl_d, scl.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
-        return seg_scale_by(es, n, B, scl_d, 0.0, s);
+    auto normalize = [&](double* B) -> qsb_status {
+        // Normalize (source/vecmath.h:128-134): x /= sqrt(|x|^2 dV); a zero or non-finite band
+        // shows in the Rayleigh quotients below
+        QSB_TRY(seg_norms(es, n, B, dVol, xn_d, sx_d, s));
+        return seg_scale_by(es, n, B, sx_d, 0.0, s);
     };
 
     // initial residual (:63-90)
-    QSB_TRY(normalize(X, nullptr));
+    QSB_TRY(normalize(X));
     QSB_TRY(apply_op(es, n, X, es->AX, s));
     if (is_first_time) {
         QSB_CUDA_TRY(cudaMemsetAsync(keep, 0, sizeof(double) * L * n, s));
@@ -1609,7 +1694,7 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     }
     QSB_TRY(seg_dot(es, n, X, es->AX, dVol, eps_d, s));
     QSB_TRY(seg_residual(es, n, es->R, es->AX, X, eps_d, nullptr, 1.0, s));
-    QSB_TRY(normalize(es->R, nullptr));
+    QSB_TRY(normalize(es->R));
     std::vector<double> eps(n);
     QSB_TRY(host_vec(eps_d, eps));
     for (int k = 0; k < n; ++k) eigen_values[k] = eps[k];
@@ -1622,43 +1707,41 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
         const int m = nblk * n;
         const double* U[3] = {X, es->R, keep};
         const double* AU[3] = {es->AX, es->AR, es->AP};
-        for (int I = 0; I < nblk; ++I)
-            for (int J = I; J < nblk; ++J) {
-                QSB_TRY(gram_block(es, U[I], AU[J], n, es->Sa, m, I, J, dVol, s));
-                QSB_TRY(gram_block(es, U[I], U[J], n, es->Sb, m, I, J, dVol, s));
-            }
+        if (es->gsmall) {
+            QSB_TRY(gram_small(es->N, n, nblk, U, AU, dVol, es->Sa, es->Sb, es->gsmall, s));
+        } else {
+            for (int I = 0; I < nblk; ++I)
+                for (int J = I; J < nblk; ++J) {
+                    QSB_TRY(gram_block(es, U[I], AU[J], n, es->Sa, m, I, J, dVol, s));
+                    QSB_TRY(gram_block(es, U[I], U[J], n, es->Sb, m, I, J, dVol, s));
+                }
+        }
         QSB_TRY(solve_pencil_fp64(es, m, n, s));   // DSYGVX, lowest n (:209, :284)
         QSB_TRY(make_coefficients(es, n, m, nblk, s));
-        // P = R Cr (+ P Cp); X = X Cx + P; same for A-bundles (:226-365)
+        // P = R Cr (+ P Cp); X = X Cx + P; same for A-bundles (:226-365), each renormalised
+        // as it leaves TMP (x, p and with their factors Ax, Ap, :493-505), and eps = <x|Ax> dV
+        // (:507) taken in Ax's pass.  The norms stay on the device until the iteration's end.
         QSB_TRY(rotate_real(es, n, es->TMP, es->R, 1, 0.0, s));
         if (!two) QSB_TRY(rotate_real(es, n, es->TMP, keep, 2, 1.0, s));
-        QSB_CUDA_TRY(cudaMemcpyAsync(keep, es->TMP, sizeof(double) * L * n, cudaMemcpyDeviceToDevice, s));
+        QSB_TRY(seg_norms(es, n, es->TMP, dVol, pn_d, sp_d, s));
+        QSB_TRY(seg_scaled_copy(es, n, es->TMP, keep, sp_d, nullptr, 0.0, nullptr, s));
         QSB_TRY(rotate_real(es, n, es->TMP, X, 0, 1.0, s));
-        QSB_CUDA_TRY(cudaMemcpyAsync(X, es->TMP, sizeof(double) * L * n, cudaMemcpyDeviceToDevice, s));
+        QSB_TRY(seg_norms(es, n, es->TMP, dVol, xn_d, sx_d, s));
+        QSB_TRY(seg_scaled_copy(es, n, es->TMP, X, sx_d, nullptr, 0.0, nullptr, s));
         QSB_TRY(rotate_real(es, n, es->TMP, es->AR, 1, 0.0, s));
         if (!two) QSB_TRY(rotate_real(es, n, es->TMP, es->AP, 2, 1.0, s));
-        QSB_CUDA_TRY(cudaMemcpyAsync(es->AP, es->TMP, sizeof(double) * L * n, cudaMemcpyDeviceToDevice, s));
+        QSB_TRY(seg_scaled_copy(es, n, es->TMP, es->AP, sp_d, nullptr, 0.0, nullptr, s));
         QSB_TRY(rotate_real(es, n, es->TMP, es->AX, 0, 1.0, s));
-        QSB_CUDA_TRY(cudaMemcpyAsync(es->AX, es->TMP, sizeof(double) * L * n, cudaMemcpyDeviceToDevice, s));
-        // renormalize x, p and Ax, Ap (:493-505)
-        std::vector<double> sx(n), sp(n);
-        QSB_TRY(seg_dot(es, n, X, X, dVol, nrm_d, s));
-        QSB_TRY(host_vec(nrm_d, v));
-        for (int k = 0; k < n; ++k) sx[k] = 1.0 / std::sqrt(v[k]);
-        QSB_TRY(seg_dot(es, n, keep, keep, dVol, nrm_d, s));
-        QSB_TRY(host_vec(nrm_d, v));
-        for (int k = 0; k < n; ++k) sp[k] = 1.0 / std::sqrt(v[k]);
-        QSB_CUDA_TRY(cudaMemcpyAsync(scl_d, sx.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
-        QSB_TRY(seg_scale_by(es, n, X, scl_d, 0.0, s));
-        QSB_TRY(seg_scale_by(es, n, es->AX, scl_d, 0.0, s));
-        QSB_CUDA_TRY(cudaMemcpyAsync(scl_d, sp.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
-        QSB_TRY(seg_scale_by(es, n, keep, scl_d, 0.0, s));
-        QSB_TRY(seg_scale_by(es, n, es->AP, scl_d, 0.0, s));
-        // eps = <x|Ax> dV; r = Ax - eps x; ||r||^2 dV (:507-513)
-        QSB_TRY(seg_dot(es, n, X, es->AX, dVol, eps_d, s));
+        QSB_TRY(seg_scaled_copy(es, n, es->TMP, es->AX, sx_d, X, dVol, eps_d, s));
+        // r = Ax - eps x; ||r||^2 dV (:507-513)
         QSB_TRY(seg_residual(es, n, es->R, es->AX, X, eps_d, nrm_d, dVol, s));
-        QSB_TRY(host_vec(eps_d, eps));
-        QSB_TRY(host_vec(nrm_d, v));
+        std::vector<double> all(4 * (size_t)n);      // eps, |r|^2, |x|^2, |p|^2
+        QSB_CUDA_TRY(cudaMemcpyAsync(all.data(), es->vec, sizeof(double) * all.size(), cudaMemcpyDeviceToHost, s));
+        QSB_CUDA_TRY(cudaStreamSynchronize(s));
+        for (double q : all)
+            if (!std::isfinite(q)) return fail(QSB_ERR_NUMERIC, "lobpcg_d: non-finite value");
+        std::copy(all.begin(), all.begin() + n, eps.begin());
+        std::copy(all.begin() + n, all.begin() + 2 * n, v.begin());
         double rmax = 0.0;
         for (int k = 0; k < n; ++k) {
             eigen_values[k] = eps[k];

@@ -191,6 +191,12 @@ qsb_status nl_apply(qsb_dtype dt, const NLDevice& d, int N, int nb, int is_compl
 bool pencil_small_fits(int m, int n, bool cplx);
 qsb_status pencil_small(int m, int n, bool cplx, double* Sa, double* Sb, double* W, int* info, cudaStream_t s);
 
+// Real pencil A = scale U^T AU, B = scale U^T U of nblk bundles of n bands each in two
+// launches (gram_small.cu); partial: gram_small_doubles(n) doubles, 0 when 3 n is too many.
+size_t gram_small_doubles(int n);
+qsb_status gram_small(int64_t N, int n, int nblk, const double* const* U, const double* const* AU, double scale,
+                      double* A, double* B, double* partial, cudaStream_t s);
+
 // Split-BF16x3 tensor-core Gram products (gram_tc.cu).
 //
 // A tall operand is a set of columns of N grid values (fp32 or fp64, one
