@@ -16,9 +16,10 @@
 // the rotation X' = X Cx + R Cr + P Cp is the two-DGEMM "conj / rot"
 // real-view product of NextVector_z2 (:1515-1598).  Band-wise reductions are
 // deterministic two-pass kernels (fixed-order partial sums, no atomics).
-// Every Gram block is recomputed each iteration (the reference does so on the
-// first and every 6th iteration, :2093; in between it updates some blocks
-// from the eigenvectors, NextMatrix_z_blasmp).
+// The real FP64 pencil is formed whole, in gram_small.cu (up to 32 bands) or
+// gram_i8_f64.cu.  The complex solver recomputes every block on the first and
+// every 6th iteration and updates some from the eigenvectors in between
+// (NextMatrix_z_blasmp, :2093); the real one recomputes all of them always.
 #include "qsb_internal.h"
 
 #include <cublas_v2.h>
@@ -308,6 +309,8 @@ struct qsb_eigensolver {
     double* vec = nullptr;           // small per-band vectors (eps, norms, scales): 8 x nmax
     double* partial = nullptr;       // reduction partials: nmax x nch
     double* gsmall = nullptr;        // tiles of the small real pencil (gram_small), few bands only
+    void* gi8 = nullptr;             // workspace of the large real pencil (gram_f64_i8), many bands only
+    size_t gi8_bytes = 0;
     int nch = 0, chunk = 0;          // pieces of a band in the reductions, elements per piece
     void* swork = nullptr;
     int slwork = 0;
@@ -1314,6 +1317,13 @@ qsb_status qsb_eigensolver_create_ex(qsb_eigensolver** out, int64_t N, int n, in
     if (!es->mixed && !is_complex && gram_small_doubles(n) > 0 &&
         cudaMalloc((void**)&es->gsmall, gram_small_doubles(n) * sizeof(double)) != cudaSuccess)
         return cleanup(fail(QSB_ERR_NOMEM, "eigensolver: pencil tile allocation"));
+    if (!es->mixed && !is_complex && gram_f64_i8_bytes(N, n) > 0) {
+        es->gi8_bytes = gram_f64_i8_bytes(N, n);
+        if (cudaMalloc(&es->gi8, es->gi8_bytes) != cudaSuccess) {
+            cudaGetLastError();          // without it the blocks are DGEMMs
+            es->gi8 = nullptr;
+        }
+    }
     if (!es->mixed && is_complex) {
         const size_t mx = (size_t)3 * n;
         if (cudaMalloc((void**)&es->nxt, sizeof(double2) * (2 * mx * mx + (size_t)6 * n * n + 2 * mx * n)) !=
@@ -1350,7 +1360,8 @@ qsb_status qsb_eigensolver_destroy(qsb_eigensolver* es) {
     float* b32[7] = {es->X32, es->R32, es->P32, es->AX32, es->AR32, es->AP32, es->TMP32};
     for (float* p : b32)
         if (p) cudaFree(p);
-    void* mw[10] = {es->su, es->sau, es->gpart, es->T2, es->rc32, es->svq, es->rotw, es->rotc, es->nxt, es->gsmall};
+    void* mw[11] = {es->su,   es->sau,  es->gpart, es->T2,     es->rc32, es->svq,
+                    es->rotw, es->rotc, es->nxt,   es->gsmall, es->gi8};
     for (void* p : mw)
         if (p) cudaFree(p);
     if (es->T) cudaFree(es->T);
@@ -1699,6 +1710,8 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     QSB_TRY(host_vec(eps_d, eps));
     for (int k = 0; k < n; ++k) eigen_values[k] = eps[k];
 
+    const size_t gi8_need = es->gi8 ? gram_f64_i8_bytes(es->N, n) : 0;   // of these n bands
+    const bool gi8 = gi8_need > 0 && gi8_need <= es->gi8_bytes;
     int iter;
     for (iter = 0; iter < iter_max; ++iter) {
         QSB_TRY(apply_op(es, n, es->R, es->AR, s));
@@ -1709,6 +1722,8 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
         const double* AU[3] = {es->AX, es->AR, es->AP};
         if (es->gsmall) {
             QSB_TRY(gram_small(es->N, n, nblk, U, AU, dVol, es->Sa, es->Sb, es->gsmall, s));
+        } else if (gi8) {
+            QSB_TRY(gram_f64_i8(es->N, n, nblk, U, AU, dVol, es->Sa, es->Sb, es->gi8, es->gi8_bytes, s));
         } else {
             for (int I = 0; I < nblk; ++I)
                 for (int J = I; J < nblk; ++J) {

@@ -1,6 +1,6 @@
 """The small real pencil formed in two launches (gram_small.cu), through the first
 step of the real FP64 solver, at band counts around its tiles and limit (33 and
-more bands take the DGEMM blocks) and grids around its 64-point chunks.
+more bands take gram_i8_f64.cu) and grids around its 64-point chunks.
 
 One iteration from dV-orthonormal bands: the Ritz values of span{X, R} against
 numpy's (1e-11 relative to the largest: sums of at most 1e4 terms and the pencil's
