@@ -1037,7 +1037,7 @@ qsb_status nl_upload(NLDevice& d, int nx, int ny, int nz, int n_atoms, const int
     std::vector<int> cptr(1, 0), catoms, e_local(total);
     d.max_local = 0;
     {
-        std::vector<int> seen(n_atoms, -1), here;
+        std::vector<int> seen(n_atoms, -1), place(n_atoms), here;
         for (size_t r0 = 0; r0 < cov.size(); r0 += APPLY_THREADS) {
             const size_t r1 = std::min(cov.size(), r0 + (size_t)APPLY_THREADS);
             here.clear();
@@ -1048,9 +1048,8 @@ qsb_status nl_upload(NLDevice& d, int nx, int ny, int nz, int n_atoms, const int
                         here.push_back(e_atom[e]);
                     }
             std::sort(here.begin(), here.end());
-            for (size_t r = r0; r < r1; ++r)
-                for (int e = gptr[cov[r]]; e < gptr[cov[r] + 1]; ++e)
-                    e_local[e] = (int)(std::lower_bound(here.begin(), here.end(), e_atom[e]) - here.begin());
+            for (size_t i = 0; i < here.size(); ++i) place[here[i]] = (int)i;
+            for (int e = gptr[cov[r0]]; e < gptr[cov[r1 - 1] + 1]; ++e) e_local[e] = place[e_atom[e]];
             catoms.insert(catoms.end(), here.begin(), here.end());
             cptr.push_back((int)catoms.size());
             d.max_local = std::max(d.max_local, (int)here.size());
