@@ -21,6 +21,7 @@
 //    (mCreateNonoverlapList, :3410-3487), and the pull can be fused into the H
 //    stencil so Hpsi is written once.
 #include "qsb_internal.h"
+#include "apply_schedule.h"
 #include <cmath>
 #include <algorithm>
 #include <numeric>
@@ -619,11 +620,9 @@ template <typename T, bool CPLX>
 struct ApplyCfg {
     static constexpr bool DIRECT = sizeof(T) == 8 && !CPLX;
     static constexpr int SG = DIRECT ? 16 : 8;               // columns per group
-    // groups in the ring; a slice's copies, issued with the first group of the slice before, are
-    // complete when it starts if S <= groups per slice + 1
-    static constexpr int S = DIRECT ? 0 : (sizeof(T) == 8 ? 3 : 5);
+    static constexpr int S = DIRECT ? 0 : (sizeof(T) == 8 ? 3 : 5);   // groups in the ring
     static constexpr int RING = S * SG * APPLY_THREADS * (int)sizeof(T);
-    static_assert(S <= APPLY_CW / SG + 1, "a slice must be complete before its first group");
+    using Order = ApplySchedule<S, APPLY_CW / SG>;           // when which copies are committed and waited for
 };
 
 // doubles of one atom's rows in a slice: 16 bytes of padding keep two atoms' rows in different banks
@@ -641,7 +640,7 @@ nl_apply_ring_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __r
     extern __shared__ __align__(16) unsigned char apply_sm[];   // ring [S][SG][256] T, then 2 coefficient slices
     constexpr int MAXE = WM <= 4 ? 3 : 1;                       // entries kept in registers
     using CF = ApplyCfg<T, CPLX>;
-    constexpr int SG = CF::SG, S = CF::S;
+    constexpr int SG = CF::SG, S = CF::S, PROLOGUE = CF::Order::PROLOGUE;
     constexpr int STAGE = SG * APPLY_THREADS * (int)sizeof(T);
     const int arow = apply_row(wmax);
     double* csm = reinterpret_cast<double*>(apply_sm + CF::RING);
@@ -680,9 +679,10 @@ nl_apply_ring_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __r
                 if (k < kc) cp_async<(int)sizeof(T)>(dst + (uint32_t)(k * APPLY_THREADS * (int)sizeof(T)), src);
         }
     };
+    // slice 0 is in the first committed group, with or without a ring
     slice(0);
 #pragma unroll
-    for (int n = 0; n < S - 1; ++n) {
+    for (int n = 0; n < PROLOGUE; ++n) {
         issue(n);
         cp_commit();
     }
@@ -758,12 +758,12 @@ nl_apply_ring_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __r
     };
     for (int n = 0; n < groups; ++n) {
         const int sl = n / (APPLY_CW / SG);
-        cp_wait<(CF::DIRECT ? 0 : S - 2)>();    // groups up to n have landed (this thread's copies)
+        cp_wait<CF::Order::PENDING>();      // groups up to n have landed (this thread's copies)
         if (n % (APPLY_CW / SG) == 0) {
             __syncthreads();                // slice sl is whole, slice sl - 1 is no longer read
             if ((sl + 1) * APPLY_CW < ncol) slice(sl + 1);
         }
-        issue(n + S - 1);
+        issue(n + PROLOGUE);
         cp_commit();
         if (!active) continue;
         const int kc = min(SG, ncol - n * SG);
