@@ -22,6 +22,7 @@ def _case(n=16, a=6.0, shift=0.07):
     return grid, pos, [dict(O.GTH_BCC)] * len(pos)
 
 
+@pytest.mark.skipif(not O.ref_available(), reason="oracle/_ref not built")
 @pytest.mark.parametrize("cplx,g", [(False, (0.0, 0.0, 0.0)), (True, (0.3, 0.2, -0.1))])
 def test_oracle_energy_force_matches_reference(cplx, g):
     grid, pos, sps = _case()
