@@ -104,7 +104,8 @@ __global__ void seg_finalize(const double* __restrict__ partial, int nseg, int n
     out[s] = t * scale;
 }
 
-// sums as seg_finalize, and their inverse square roots
+// sums as seg_finalize, and their inverse square roots (1 where the sum is not finite: the
+// band stays as it is and the host refuses the call by the sum)
 __global__ void seg_finalize_rsqrt(const double* __restrict__ partial, int nseg, int nch, double scale,
                                    double* __restrict__ out, double* __restrict__ inv) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -112,7 +113,7 @@ __global__ void seg_finalize_rsqrt(const double* __restrict__ partial, int nseg,
     double t = 0.0;
     for (int c = 0; c < nch; ++c) t += partial[(size_t)s * nch + c];
     out[s] = t * scale;
-    inv[s] = 1.0 / sqrt(t * scale);
+    inv[s] = isfinite(t * scale) ? 1.0 / sqrt(t * scale) : 1.0;
 }
 
 // out[s] = in[s] * scale[s] and, with partial, partial sums of out[s] * y[s] in
@@ -1704,22 +1705,20 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     double* sp_d = es->vec + 5 * n;
     std::vector<double> v(n);
 
-    auto host_vec = [&](const double* d, std::vector<double>& h) -> qsb_status {
-        QSB_CUDA_TRY(cudaMemcpyAsync(h.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+    auto to_host = [&](std::vector<double>& h) -> qsb_status {      // the first h.size() of es->vec
+        QSB_CUDA_TRY(cudaMemcpyAsync(h.data(), es->vec, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s));
         QSB_CUDA_TRY(cudaStreamSynchronize(s));
-        for (int k = 0; k < n; ++k)
-            if (!std::isfinite(h[k])) return fail(QSB_ERR_NUMERIC, "lobpcg_d: non-finite value");
         return QSB_OK;
     };
-    auto normalize = [&](double* B) -> qsb_status {
-        // Normalize (source/vecmath.h:128-134): x /= sqrt(|x|^2 dV); a zero or non-finite band
-        // shows in the Rayleigh quotients below
-        QSB_TRY(seg_norms(es, n, B, dVol, xn_d, sx_d, s));
+    auto normalize = [&](double* B, double* norms) -> qsb_status {
+        // Normalize (source/vecmath.h:128-134): x /= sqrt(|x|^2 dV); the norms are looked at
+        // in the wait for the Rayleigh quotients below
+        QSB_TRY(seg_norms(es, n, B, dVol, norms, sx_d, s));
         return seg_scale_by(es, n, B, sx_d, 0.0, s);
     };
 
     // initial residual (:63-90)
-    QSB_TRY(normalize(X));
+    QSB_TRY(normalize(X, xn_d));
     QSB_TRY(apply_op(es, n, X, es->AX, s));
     if (is_first_time) {
         QSB_CUDA_TRY(cudaMemsetAsync(keep, 0, sizeof(double) * L * n, s));
@@ -1729,9 +1728,18 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     }
     QSB_TRY(seg_dot(es, n, X, es->AX, dVol, eps_d, s));
     QSB_TRY(seg_residual(es, n, es->R, es->AX, X, eps_d, nullptr, 1.0, s));
-    QSB_TRY(normalize(es->R));
+    QSB_TRY(normalize(es->R, pn_d));
     std::vector<double> eps(n);
-    QSB_TRY(host_vec(eps_d, eps));
+    {
+        // an infinite |x|^2 or |r|^2 (its band finite, so the quotients can be) is refused here as
+        // any other: the pencil of such a band is NaN
+        std::vector<double> first(4 * (size_t)n);       // eps, (not yet written), |x|^2, |r|^2
+        QSB_TRY(to_host(first));
+        for (int k = 0; k < n; ++k)
+            if (!std::isfinite(first[k]) || !std::isfinite(first[2 * n + k]) || !std::isfinite(first[3 * n + k]))
+                return fail(QSB_ERR_NUMERIC, "lobpcg_d: non-finite value");
+        std::copy(first.begin(), first.begin() + n, eps.begin());
+    }
     for (int k = 0; k < n; ++k) eigen_values[k] = eps[k];
 
     const size_t gi8_need = es->gi8 ? gram_f64_i8_bytes(es->N, n) : 0;   // of these n bands
@@ -1775,8 +1783,7 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
         // r = Ax - eps x; ||r||^2 dV (:507-513)
         QSB_TRY(seg_residual(es, n, es->R, es->AX, X, eps_d, nrm_d, dVol, s));
         std::vector<double> all(4 * (size_t)n);      // eps, |r|^2, |x|^2, |p|^2
-        QSB_CUDA_TRY(cudaMemcpyAsync(all.data(), es->vec, sizeof(double) * all.size(), cudaMemcpyDeviceToHost, s));
-        QSB_CUDA_TRY(cudaStreamSynchronize(s));
+        QSB_TRY(to_host(all));
         for (double q : all)
             if (!std::isfinite(q)) return fail(QSB_ERR_NUMERIC, "lobpcg_d: non-finite value");
         std::copy(all.begin(), all.begin() + n, eps.begin());
