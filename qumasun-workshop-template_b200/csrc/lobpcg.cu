@@ -339,7 +339,7 @@ struct qsb_eigensolver {
     int nch = 0, chunk = 0;          // pieces of a band in the reductions, elements per piece
     void* swork = nullptr;
     int slwork = 0;
-    int* info = nullptr;
+    int* info = nullptr;             // [0] of the dense solves, [1] non-zero: the pencil's products gave up
     // operator
     qsb_ham* ham = nullptr;
     double g[3] = {0, 0, 0};
@@ -1371,7 +1371,7 @@ qsb_status qsb_eigensolver_create_ex(qsb_eigensolver** out, int64_t N, int n, in
     es->rc = es->W + m;
     es->vec = es->rc + (size_t)6 * 2 * n * n;
     es->partial = es->vec + 8 * (size_t)n;
-    if (cudaMalloc((void**)&es->info, sizeof(int)) != cudaSuccess)
+    if (cudaMalloc((void**)&es->info, 2 * sizeof(int)) != cudaSuccess)
         return cleanup(fail(QSB_ERR_NOMEM, "eigensolver: info allocation"));
     *out = es;
     return QSB_OK;
@@ -1743,7 +1743,7 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     for (int k = 0; k < n; ++k) eigen_values[k] = eps[k];
 
     const size_t gi8_need = es->gi8 ? gram_f64_i8_bytes(es->N, n) : 0;   // of these n bands
-    const bool gi8 = gi8_need > 0 && gi8_need <= es->gi8_bytes;
+    bool gi8 = gi8_need > 0 && gi8_need <= es->gi8_bytes;
     int iter;
     for (iter = 0; iter < iter_max; ++iter) {
         QSB_TRY(apply_op(es, n, es->R, es->AR, s));
@@ -1755,8 +1755,18 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
         if (es->gsmall) {
             QSB_TRY(gram_small(es->N, n, nblk, U, AU, dVol, es->Sa, es->Sb, es->gsmall, s));
         } else if (gi8) {
-            QSB_TRY(gram_f64_i8(es->N, n, nblk, U, AU, dVol, es->Sa, es->Sb, es->gi8, es->gi8_bytes, s));
-        } else {
+            QSB_CUDA_TRY(cudaMemsetAsync(es->info + 1, 0, sizeof(int), s));
+            QSB_TRY(gram_f64_i8(es->N, n, nblk, U, AU, dVol, es->Sa, es->Sb, es->gi8, es->gi8_bytes, es->info + 1, s));
+            // the products' waits are bounded: a pencil that they did not finish is formed
+            // by the library instead, here and for the rest of the call (the device error
+            // word says so too).  Looked at before anything is solved: the library's dense
+            // solvers may never come back from a pencil of zeros.
+            int gave_up = 0;
+            QSB_CUDA_TRY(cudaMemcpyAsync(&gave_up, es->info + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+            QSB_CUDA_TRY(cudaStreamSynchronize(s));
+            gi8 = gave_up == 0;
+        }
+        if (!es->gsmall && !gi8) {
             for (int I = 0; I < nblk; ++I)
                 for (int J = I; J < nblk; ++J) {
                     QSB_TRY(gram_block(es, U[I], AU[J], n, es->Sa, m, I, J, dVol, s));

@@ -204,7 +204,7 @@ qsb_status gram_small(int64_t N, int n, int nblk, const double* const* U, const 
 constexpr int GRAM_F64_I8_MIN_BANDS = 33;
 size_t gram_f64_i8_bytes(int64_t N, int n);
 qsb_status gram_f64_i8(int64_t N, int n, int nblk, const double* const* U, const double* const* AU, double scale,
-                       double* A, double* B, void* ws, size_t ws_bytes, cudaStream_t s);
+                       double* A, double* B, void* ws, size_t ws_bytes, int* gave_up, cudaStream_t s);
 
 // Split-BF16x3 tensor-core Gram products (gram_tc.cu).
 //
