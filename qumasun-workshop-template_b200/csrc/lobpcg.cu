@@ -339,7 +339,7 @@ struct qsb_eigensolver {
     int nch = 0, chunk = 0;          // pieces of a band in the reductions, elements per piece
     void* swork = nullptr;
     int slwork = 0;
-    int* info = nullptr;             // [0] of the dense solves, [1] non-zero: the pencil's products gave up
+    int* info = nullptr;             // [0] of the dense solves, [1] of the pencil's products and its look-over
     // operator
     qsb_ham* ham = nullptr;
     double g[3] = {0, 0, 0};
@@ -511,9 +511,37 @@ qsb_status gram_block(qsb_eigensolver* es, const double* U, const double* V, int
     return QSB_OK;
 }
 
+// state |= 1: an entry of the pencil (n doubles each) is not finite, 2: a diagonal entry of
+// B (every dstep-th) is not positive
+__global__ void pencil_state(const double* __restrict__ A, const double* __restrict__ B, size_t n, size_t dstep,
+                             int* __restrict__ state) {
+    int bad = 0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const double a = A[i], b = B[i];
+        if (!isfinite(a) || !isfinite(b)) bad |= 1;
+        if (i % dstep == 0 && !(b > 0.0)) bad |= 2;
+    }
+    if (bad) atomicOr(state, bad);
+}
+
 // generalized eigenproblem Sa c = lambda Sb c (m x m), eigenvalues ascending into
 // es->W, eigenvectors into Sa (B-orthonormal).
 qsb_status solve_pencil(qsb_eigensolver* es, int m, cudaStream_t s) {
+    // The library's solvers may never come back from a pencil with an entry that is not finite
+    // (observed: from one of zeros, whose reduction divides by zero): such a pencil is refused,
+    // one with a vanishing column of B is not positive definite.
+    {
+        const size_t c2 = es->cplx ? 2 : 1, cnt = (size_t)m * m * c2;
+        int state = 0;
+        QSB_CUDA_TRY(cudaMemsetAsync(es->info + 1, 0, sizeof(int), s));
+        pencil_state<<<(int)std::min<size_t>((cnt + 255) / 256, 512), 256, 0, s>>>(es->Sa, es->Sb, cnt,
+                                                                                  ((size_t)m + 1) * c2, es->info + 1);
+        QSB_CUDA_TRY(cudaGetLastError());
+        QSB_CUDA_TRY(cudaMemcpyAsync(&state, es->info + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+        QSB_CUDA_TRY(cudaStreamSynchronize(s));
+        if (state & 1) return fail(QSB_ERR_NUMERIC, "eigensolver: non-finite pencil");
+        if (state & 2) return fail(QSB_ERR_SOLVER, "eigensolver: generalized eigenproblem failed (overlap matrix not positive definite)");
+    }
     int lwork = 0;
     if (es->cplx) {
         QSB_SOLVER_TRY(cusolverDnZhegvd_bufferSize(es->sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR,
@@ -823,7 +851,9 @@ qsb_status solve_pencil_overlap_basis(qsb_eigensolver* es, int m, int nout, cuda
         QSB_CUDA_TRY(cudaMemcpyAsync(Wm, es->Sa, sizeof(double) * mm, cudaMemcpyDeviceToDevice, s));
         QSB_CUDA_TRY(cudaMemcpyAsync(tmp, es->Sb, sizeof(double) * mm, cudaMemcpyDeviceToDevice, s));
         const std::string saved_error = qsb_last_error();
-        if (solve_pencil(es, m, s) == QSB_OK) {
+        const qsb_status st = solve_pencil(es, m, s);
+        if (st == QSB_ERR_NUMERIC) return st;
+        if (st == QSB_OK) {
             rows_scale<<<dim3((m + 127) / 128, nout), 128, 0, s>>>(es->Sa, d, m, nout, es->cplx, es->Sa);
             QSB_CUDA_TRY(cudaGetLastError());
             ++es->last_chol;
