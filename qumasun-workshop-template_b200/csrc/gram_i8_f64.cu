@@ -1,34 +1,44 @@
 // The real FP64 Rayleigh-Ritz pencil of many bands on the INT8 tensor cores: all
 // upper tiles of S = dV U^T U and A = dV U^T (AU), U = [X R P] gathered columns,
-// with more bits than an FP64 product sum keeps.
+// from products that are exact up to a fixed fraction of the columns' maxima.
 //
 // Splitting: column c becomes integers x = rint(u 2^e_c), 2^54 <= max |x| < 2^55,
 // each written as seven balanced base-256 digits
 //   x = sum_i d_i 256^(6-i),  -128 <= d_i <= 127.
 //   U^T V = 2^(-e_u - e_v) sum_l 256^(12-l) D_l,  D_l = sum_{i+j=l} d_i^T d'_j
-// The 34 products with i + j <= 7 are summed without rounding in INT32
-// (7 * 2^14 * K < 2^31 for the at most 18688 points of a CTA), a level at a time.
-// Of the omitted products, below 2^-64 of the columns' maxima, only those of
-// equal digits have one sign.  Largest error of the entries relative to |u||v|,
-// against twice-FP64 sums: 1.1e-16 to 4.6e-16, where the library's products have
-// 5e-16 to 1.9e-14; root mean square 0.1 to 0.3 of theirs or less (25^3 to 96^3
-// points, random, plane-wave-like and localised columns; without the level i + j =
-// 7 the localised ones were 3 times worse than the library's in the mean).
+// The 34 products with i + j <= 7 and the product d_4^T d'_4 are summed without
+// rounding in INT32 (7 * 2^14 * K < 2^31 for the at most 18688 points of a CTA), a
+// level at a time.
+//
+// Precision: what is kept is relative to a column's largest value, not to each
+// element: an element below a quarter of it has fewer bits here than in FP64, with
+// an error of at most 2^-55 max|u|.  The products left out are each below 2^-64 of
+// max|u| max|v| at a point.  Their signs alternate from point to point, except where
+// a column meets itself (or its double) digit on equal digit: sum d_4^2, without which
+// <u|u> of a column with one dominant point was low by N 2^-66, 5e-14 at 96^3 and
+// 2e-13 at 144^3, is therefore one of the products; the next, sum d_5^2, is below
+// N 2^-82.  Errors of entries relative to |u||v| in exact integers at 96^3 and 144^3:
+//   one point at 1, the others uniform within 1e-2 to 1e-6, or a Gaussian one
+//     grid spacing wide on a tail of 1e-4:        at most 4e-16 (FP64 sums up to 6e-15)
+//   the others within 10 % of one value:           at most 3e-15 (9e-15)
+//   uniform, waves, wide Gaussians, exponentials: at most 3e-17 (1e-14)
+//   one point at 1, all others the same number (signs alternate nowhere):
+//                                                 up to 3e-13 (6e-13; 5e-16 where the
+//                                                 partner's digits do vary, 5e-14 here)
 //
 // Why: the FP64 units give 37 TFLOP/s, and a library product of 128 x 128 columns
 // over 96^3 points, 29 GFLOP, takes 1.0 ms; a pencil of 384 columns is 12 of them,
 // three with a lower triangle that no one needs.  Pencil of 3 n columns, library ->
-// here: n = 128, 96^3 12.9 -> 6.5 ms (maxima 0.7, digits 1.7, products 3.4); n = 200,
-// 64^3 11.6 -> 4.1; n = 48, 96^3 3.8 -> 3.3 (144 columns are padded to 256); n = 33,
-// 32^3 0.25 -> 0.11 ms.  The digits are bound by their 15 bytes moved per element, the
+// here: n = 128, 96^3 12.9 -> 6.7 ms (maxima 0.8, digits 1.7, products 4.2); n = 200,
+// 64^3 11.6 -> 4.5; n = 48, 96^3 3.8 -> 3.0 (144 columns are padded to 256); n = 33,
+// 32^3 0.25 -> 0.14 ms.  The digits are bound by their 15 bytes moved per element, the
 // products by the integer MMA rate and, in the second launch, by the operands' way
 // from L2 to shared memory.
 //
 // The digits of one chunk of grid points are laid out at a time (bounded
-// workspace), [digit][column][point]; a chunk takes two launches of CTAs with 128
-// x 128 output tiles, one for the levels 4 to 7 and one for 0 to 3, because the
-// INT32 accumulators of eight levels (128 TMEM columns each) do not fit the 512
-// columns of an SM.  Pipeline per CTA as in gram_i8.cu: warp 0 lane 0 streams
+// workspace), [digit][column][point]; a chunk takes three launches of CTAs with 128
+// x 128 output tiles, for d_4 d'_4, the levels 4 to 7 and 0 to 3, because no more
+// than four INT32 accumulators (128 TMEM columns each) fit the 512 columns of an SM.  Pipeline per CTA as in gram_i8.cu: warp 0 lane 0 streams
 // 64-point stages of the digit tiles with 2-D TMA copies (64-byte swizzle), warp 1
 // lane 0 issues the MMAs, the four warps combine the levels into FP64 partial
 // tiles.  All waits are bounded; a wait that runs out sets the device error word
@@ -51,18 +61,28 @@ constexpr int GF_THREADS = 128;
 constexpr int GF_MAX_STAGES = 18688 / GF_K;      // 7 * 128 * 128 * 18688 < 2^31
 constexpr unsigned GF_WAIT_LIMIT = 1u << 22;
 constexpr unsigned GF_DRAIN_LIMIT = 1u << 16;
+constexpr int GF_PASSES = 3;                     // launches per chunk of points
 constexpr int ERR_GEMM_TIMEOUT = 2;
 constexpr size_t GF_DIGIT_BYTES = (size_t)1 << 30;   // most digits laid out at a time
 
-// One launch: the levels LO..HI from digits 0..min(HI, 6) of both operands
-template <int LO, int HI>
+// One launch: the products of levels LO..HI of the digits FIRST..LAST of both operands
+template <int LO, int HI, int FIRST, int LAST>
 struct GfPass {
-    static constexpr int digits = HI < GF_DIGITS ? HI + 1 : GF_DIGITS;
-    static constexpr int stages = digits == GF_DIGITS ? 2 : 3;
+    static_assert(HI - LO < 4, "four accumulators of 128 TMEM columns");
+    static constexpr int digits = LAST - FIRST + 1;
+    // (more than half of the shared memory: a CTA takes all of the SM's TMEM)
+    static constexpr int stages = digits > 4 ? 2 : (digits > 1 ? 3 : 8);
     static constexpr size_t stage_bytes = (size_t)2 * digits * GF_TILE;
     static constexpr size_t smem = stages * stage_bytes + 1024 + 256;
 };
-static_assert(GfPass<4, 7>::smem <= 232448 && GfPass<0, 3>::smem <= 232448, "stages must fit the 227 KB of a CTA");
+using GfLow = GfPass<8, 8, 4, 4>;
+using GfMid = GfPass<4, 7, 0, 6>;
+using GfTop = GfPass<0, 3, 0, 3>;
+static_assert(GfLow::smem <= 232448 && GfMid::smem <= 232448 && GfTop::smem <= 232448,
+              "stages must fit the 227 KB of a CTA");
+
+// weight of level l in units of level 0
+constexpr double gf_weight(int l) { return l == 0 ? 1.0 : gf_weight(l - 1) / 256.0; }
 
 // kind::i8: signed 8-bit A and B, signed 32-bit D, both K-major, M = N = 128
 constexpr uint32_t GF_IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GF_T >> 3) << 17) |
@@ -205,12 +225,12 @@ __device__ __forceinline__ void gf_tile_of(int t, int* mt, int* nt) {
 
 // CTA: tile blockIdx.x of [S tiles, A tiles], K split blockIdx.y of the chunk.
 // partial[((split * tiles + tile) * 128 + row) * 128 + col] = sum over the levels of D_l 256^-l
-template <int LO, int HI>
+template <int LO, int HI, int FIRST, int LAST>
 __global__ void __launch_bounds__(GF_THREADS, 1)
 gram_f64_i8_kernel(const __grid_constant__ CUtensorMap mU, const __grid_constant__ CUtensorMap mV, int p, int ntl,
                    int kstages, int ksplit, double* __restrict__ partial, int* __restrict__ err,
                    int* __restrict__ own_err) {
-    using P = GfPass<LO, HI>;
+    using P = GfPass<LO, HI, FIRST, LAST>;
     constexpr int ND = P::digits, NS = P::stages;
     extern __shared__ unsigned char gf_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)gf_raw + 1023) & ~(uintptr_t)1023);
@@ -271,9 +291,10 @@ gram_f64_i8_kernel(const __grid_constant__ CUtensorMap mU, const __grid_constant
             bar_expect_tx(&full[s], (uint32_t)((one ? 1 : 2) * ND * GF_TILE));
             // rows past the last column of a digit are the next digit's (or past the
             // array: zero); they reach only entries that no one reads
-            for (int k = 0; k < ND; ++k) tma_2d(st + k * GF_TILE, &mU, kx, k * p + mt * GF_T, &full[s]);
+            for (int k = 0; k < ND; ++k) tma_2d(st + k * GF_TILE, &mU, kx, (FIRST + k) * p + mt * GF_T, &full[s]);
             if (!one)
-                for (int k = 0; k < ND; ++k) tma_2d(st + (ND + k) * GF_TILE, mB, kx, k * p + nt * GF_T, &full[s]);
+                for (int k = 0; k < ND; ++k)
+                    tma_2d(st + (ND + k) * GF_TILE, mB, kx, (FIRST + k) * p + nt * GF_T, &full[s]);
             issued = it + 1;
         }
     } else if (warp == 1 && lane == 0) {
@@ -290,11 +311,14 @@ gram_f64_i8_kernel(const __grid_constant__ CUtensorMap mU, const __grid_constant
 #pragma unroll
             for (int kk = 0; kk < GF_K / 32; ++kk)
 #pragma unroll
-                for (int l = LO; l <= HI; ++l)
+                for (int l = LO; l <= HI; ++l) {
+                    const int i0 = l - LAST > FIRST ? l - LAST : FIRST;      // digits i and l - i, both loaded
 #pragma unroll
-                    for (int i = l < ND ? 0 : l - ND + 1; i <= l && i < ND; ++i)
-                        gf_mma(tmem + 128u * (l - LO), sw64_kmajor_desc(a + i * GF_TILE + kk * 32),
-                               sw64_kmajor_desc(b + (l - i) * GF_TILE + kk * 32), it > 0 || kk > 0 || i > (l < ND ? 0 : l - ND + 1) ? 1u : 0u);
+                    for (int i = i0; i <= l - FIRST && i <= LAST; ++i)
+                        gf_mma(tmem + 128u * (l - LO), sw64_kmajor_desc(a + (i - FIRST) * GF_TILE + kk * 32),
+                               sw64_kmajor_desc(b + (l - i - FIRST) * GF_TILE + kk * 32),
+                               it > 0 || kk > 0 || i > i0 ? 1u : 0u);
+                }
             umma_commit(&empty[s]);
         }
         umma_commit(done);
@@ -315,7 +339,7 @@ gram_f64_i8_kernel(const __grid_constant__ CUtensorMap mU, const __grid_constant
         for (int l = HI; l >= LO; --l) {             // smallest level first
             uint32_t r[32];
             tmem_ld32(tmem + lane_base + 128u * (l - LO) + (uint32_t)c0, r);
-            const double f = 1.0 / (double)(1ull << (8 * l));
+            const double f = gf_weight(l);
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = l == HI ? (double)(int)r[j] * f : fma((double)(int)r[j], f, v[j]);
         }
@@ -337,7 +361,7 @@ gram_f64_i8_kernel(const __grid_constant__ CUtensorMap mU, const __grid_constant
     }
 }
 
-// Sums a chunk's partial tiles (both passes, fixed order) onto acc [2][p][p]; the
+// Sums a chunk's partial tiles (all passes, smallest levels first) onto acc [2][p][p]; the
 // last chunk writes scale 2^(...) acc to B = S (blockIdx.z = 0) and A, with the mirror.
 __global__ void gf_reduce_kernel(const double* __restrict__ partial, int slots, int ntl, int p, bool first, bool last,
                                  const unsigned long long* __restrict__ maxbits, double scale,
@@ -424,7 +448,7 @@ GfPlan plan_gf(int64_t N, int p) {
         }
     }
     g.half = a1k((size_t)GF_DIGITS * p * g.kc);
-    g.partial = a1k((size_t)2 * g.ksplit * 2 * g.ntl * GF_T * GF_T * sizeof(double));
+    g.partial = a1k((size_t)GF_PASSES * g.ksplit * 2 * g.ntl * GF_T * GF_T * sizeof(double));
     g.bytes = 2 * g.half + g.partial + a1k((size_t)2 * p * p * sizeof(double)) +
               a1k((size_t)2 * p * sizeof(unsigned long long));
     return g;
@@ -462,10 +486,12 @@ qsb_status gram_f64_i8(int64_t N, int n, int nblk, const double* const* U, const
     const int mblocks = (int)std::min<int64_t>((N / 2 + 256) / 256, std::max(1, 4736 / (2 * p)));
     gf_absmax_kernel<<<dim3(mblocks, 2 * p), 256, 0, s>>>(b, N, maxbits);
     QSB_CUDA_TRY(cudaGetLastError());
-    auto light = gram_f64_i8_kernel<0, 3>;
-    auto heavy = gram_f64_i8_kernel<4, 7>;
-    QSB_CUDA_TRY(cudaFuncSetAttribute(light, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfPass<0, 3>::smem));
-    QSB_CUDA_TRY(cudaFuncSetAttribute(heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfPass<4, 7>::smem));
+    auto low = gram_f64_i8_kernel<8, 8, 4, 4>;
+    auto mid = gram_f64_i8_kernel<4, 7, 0, 6>;
+    auto top = gram_f64_i8_kernel<0, 3, 0, 3>;
+    QSB_CUDA_TRY(cudaFuncSetAttribute(low, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfLow::smem));
+    QSB_CUDA_TRY(cudaFuncSetAttribute(mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfMid::smem));
+    QSB_CUDA_TRY(cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfTop::smem));
     const int tiles = 2 * g.ntl;
     for (int c = 0; c < g.chunks; ++c) {
         const int64_t g0 = c * g.kc;
@@ -479,14 +505,18 @@ qsb_status gram_f64_i8(int64_t N, int n, int nblk, const double* const* U, const
         gf_digit_kernel<<<dim3(dblocks, 2 * p), 256, 0, s>>>(b, N, g0, ldk, maxbits, digits, g.half);
         QSB_CUDA_TRY(cudaGetLastError());
         const int kstages = (int)(ldk / GF_K);
-        heavy<<<dim3(tiles, g.ksplit), GF_THREADS, GfPass<4, 7>::smem, s>>>(mU, mV, p, g.ntl, kstages, g.ksplit, partial,
-                                                                           device_error_word(), gave_up);
+        const dim3 grid(tiles, g.ksplit);
+        const size_t slots = (size_t)g.ksplit * tiles * GF_T * GF_T;       // of one pass
+        int* const word = device_error_word();
+        low<<<grid, GF_THREADS, GfLow::smem, s>>>(mU, mV, p, g.ntl, kstages, g.ksplit, partial, word, gave_up);
         QSB_CUDA_TRY(cudaGetLastError());
-        light<<<dim3(tiles, g.ksplit), GF_THREADS, GfPass<0, 3>::smem, s>>>(
-            mU, mV, p, g.ntl, kstages, g.ksplit, partial + (size_t)g.ksplit * tiles * GF_T * GF_T, device_error_word(),
-            gave_up);
+        mid<<<grid, GF_THREADS, GfMid::smem, s>>>(mU, mV, p, g.ntl, kstages, g.ksplit, partial + slots, word,
+                                                           gave_up);
         QSB_CUDA_TRY(cudaGetLastError());
-        gf_reduce_kernel<<<dim3((p + 127) / 128, p, 2), 128, 0, s>>>(partial, 2 * g.ksplit, g.ntl, p, c == 0,
+        top<<<grid, GF_THREADS, GfTop::smem, s>>>(mU, mV, p, g.ntl, kstages, g.ksplit, partial + 2 * slots,
+                                                           word, gave_up);
+        QSB_CUDA_TRY(cudaGetLastError());
+        gf_reduce_kernel<<<dim3((p + 127) / 128, p, 2), 128, 0, s>>>(partial, GF_PASSES * g.ksplit, g.ntl, p, c == 0,
                                                                    c + 1 == g.chunks, maxbits, scale, acc, A, B);
         QSB_CUDA_TRY(cudaGetLastError());
     }
