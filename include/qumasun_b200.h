@@ -277,7 +277,11 @@ typedef int (*qsb_apply_fn)(void* user, int nb, const double* x_dev, double* ax_
 /* Solver context for bundles of up to n bands of N grid points (complex SoA
  * when is_complex), holding the device work bundles R, AX, AR, AP and a
  * temporary (the reference's `work`/`temporary` arenas,
- * source/lobpcg_z_multi_mpi.h:2862-2881) and the cuBLAS / cuSOLVER handles. */
+ * source/lobpcg_z_multi_mpi.h:2862-2881) and the cuBLAS / cuSOLVER handles.
+ * A real FP64 context of 33 or more bands forms its pencils in the temporary
+ * bundle; where that is small (few grid points), in up to 192 MB of its own,
+ * and without memory for those in what the temporary holds or, if that is too
+ * little, by library products (another rounding of the same sums). */
 QSB_API qsb_status qsb_eigensolver_create(qsb_eigensolver** es, int64_t N, int n, int is_complex);
 
 /* Precision of a solver context.

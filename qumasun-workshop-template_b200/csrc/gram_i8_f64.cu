@@ -29,20 +29,23 @@
 // Why: the FP64 units give 37 TFLOP/s, and a library product of 128 x 128 columns
 // over 96^3 points, 29 GFLOP, takes 1.0 ms; a pencil of 384 columns is 12 of them,
 // three with a lower triangle that no one needs.  Pencil of 3 n columns, library ->
-// here: n = 128, 96^3 12.9 -> 6.7 ms (maxima 0.8, digits 1.7, products 4.2); n = 200,
-// 64^3 11.6 -> 4.5; n = 48, 96^3 3.8 -> 3.0 (144 columns are padded to 256); n = 33,
-// 32^3 0.25 -> 0.14 ms.  The digits are bound by their 15 bytes moved per element, the
-// products by the integer MMA rate and, in the second launch, by the operands' way
-// from L2 to shared memory.
+// here: n = 128, 96^3 12.9 -> 6.8 ms (maxima 0.8, digits 1.7, products 4.3); n = 200,
+// 64^3 11.6 -> 4.9; n = 48, 96^3 3.8 -> 3.3 (144 columns are padded to 256); n = 33,
+// 32^3 0.25 -> 0.14 ms.  The digits are bound by their 15 bytes moved per element,
+// the products by the operands' way from L2 to shared memory (24 tiles of 8 KB per 64
+// points and output tile, 0.14 us each at the chip's 8.8 TB/s, against 35 products of
+// about 0.07).
 //
-// The digits of one chunk of grid points are laid out at a time (bounded
-// workspace), [digit][column][point]; a chunk takes three launches of CTAs with 128
-// x 128 output tiles, for d_4 d'_4, the levels 4 to 7 and 0 to 3, because no more
-// than four INT32 accumulators (128 TMEM columns each) fit the 512 columns of an SM.  Pipeline per CTA as in gram_i8.cu: warp 0 lane 0 streams
-// 64-point stages of the digit tiles with 2-D TMA copies (64-byte swizzle), warp 1
-// lane 0 issues the MMAs, the four warps combine the levels into FP64 partial
-// tiles.  All waits are bounded; a wait that runs out sets the device error word
-// and the caller's own word, and the CTA drains, frees TMEM and returns.
+// The digits of one chunk of grid points are laid out at a time, as many as the
+// workspace holds (the solver's temporary bundle, free while a pencil is formed),
+// [digit][column][point]; a chunk takes three launches of CTAs with 128 x 128 output
+// tiles, for d_4 d'_4, the levels 4 to 7 and 0 to 3, because no more than four INT32
+// accumulators (128 TMEM columns each) fit the 512 columns of an SM.  Pipeline per
+// CTA as in gram_i8.cu: warp 0 lane 0 streams 64-point stages of the digit tiles
+// with 2-D TMA copies (64-byte swizzle), warp 1 lane 0 issues the MMAs, the four
+// warps combine the levels into FP64 partial tiles.  All waits are bounded; a wait
+// that runs out sets the device error word and the caller's own word, and the CTA
+// drains, frees TMEM and returns.
 #include "qsb_internal.h"
 #include "tc_common.cuh"
 
@@ -64,6 +67,7 @@ constexpr unsigned GF_DRAIN_LIMIT = 1u << 16;
 constexpr int GF_PASSES = 3;                     // launches per chunk of points
 constexpr int ERR_GEMM_TIMEOUT = 2;
 constexpr size_t GF_DIGIT_BYTES = (size_t)1 << 30;   // most digits laid out at a time
+constexpr size_t GF_OWN_BYTES = (size_t)192 << 20;   // largest workspace of a solver's own
 
 // One launch: the products of levels LO..HI of the digits FIRST..LAST of both operands
 template <int LO, int HI, int FIRST, int LAST>
@@ -420,18 +424,24 @@ int64_t up128(int64_t x) { return (x + 127) / 128 * 128; }
 struct GfPlan {
     int ntl, ksplit, chunks;
     int64_t kc;                                  // points per chunk, a multiple of 128
-    size_t half, partial, bytes;                 // bytes of U's digits, of the partial tiles, in all
+    size_t half, partial, bytes;                 // bytes of U's digits, of the partial tiles, in all (0: no plan)
+    double cost;
 };
 
-// Points per chunk and K splits: whole waves of CTAs as far as the digits' bound
-// and the accumulators' range allow
-GfPlan plan_gf(int64_t N, int p) {
+// Points per chunk and K splits within `avail` bytes: whole waves of CTAs as far as
+// the workspace and the accumulators' range allow
+GfPlan plan_gf(int64_t N, int p, size_t avail) {
     GfPlan g{};
     const int t = (p + GF_T - 1) / GF_T;
     g.ntl = t * (t + 1) / 2;
-    const int64_t most = std::max<int64_t>(128, (int64_t)(GF_DIGIT_BYTES / (2 * GF_DIGITS * (size_t)p)) / 128 * 128);
-    double best = 0.0;
+    const size_t tile = (size_t)GF_T * GF_T * sizeof(double);
+    const size_t fixed = a1k((size_t)2 * p * p * sizeof(double)) + a1k((size_t)2 * p * sizeof(unsigned long long));
     for (int k = 1; k <= 148; ++k) {
+        const size_t partial = a1k((size_t)GF_PASSES * k * 2 * g.ntl * tile);
+        if (avail < partial + fixed + 2048) break;
+        const size_t room = std::min(GF_DIGIT_BYTES, avail - partial - fixed - 2048);    // 2048: a1k of both halves
+        const int64_t most = (int64_t)(room / (2 * GF_DIGITS * (size_t)p)) / 128 * 128;
+        if (most < 128) break;
         const int64_t cap = std::min<int64_t>(most, (int64_t)k * GF_MAX_STAGES * GF_K / 128 * 128);
         const int64_t chunks = (N + cap - 1) / cap, kc = up128((N + chunks - 1) / chunks);
         const int64_t stages = kc / GF_K;
@@ -440,26 +450,39 @@ GfPlan plan_gf(int64_t N, int p) {
         if (per > GF_MAX_STAGES) continue;
         // stages that the busiest SM works through, with some for each wave's fill and readout
         const double cost = (double)chunks * waves * (per + 16);
-        if (best == 0.0 || cost < best) {
-            best = cost;
+        if (g.bytes == 0 || cost < g.cost) {
+            g.cost = cost;
             g.ksplit = k;
             g.chunks = (int)chunks;
             g.kc = kc;
+            g.half = a1k((size_t)GF_DIGITS * p * kc);
+            g.partial = partial;
+            g.bytes = 2 * g.half + partial + fixed;
         }
     }
-    g.half = a1k((size_t)GF_DIGITS * p * g.kc);
-    g.partial = a1k((size_t)GF_PASSES * g.ksplit * 2 * g.ntl * GF_T * GF_T * sizeof(double));
-    g.bytes = 2 * g.half + g.partial + a1k((size_t)2 * p * p * sizeof(double)) +
-              a1k((size_t)2 * p * sizeof(unsigned long long));
     return g;
 }
 
+bool gf_takes(int n) { return n >= GRAM_F64_I8_MIN_BANDS && 6 * (int64_t)n <= 65535; }
+
 }  // namespace
 
-// Workspace of a pencil of up to 3 n columns (0: n is not for this form)
-size_t gram_f64_i8_bytes(int64_t N, int n) {
-    if (n < GRAM_F64_I8_MIN_BANDS || 6 * (int64_t)n > 65535) return 0;
-    return std::max(plan_gf(N, 2 * n).bytes, plan_gf(N, 3 * n).bytes);
+// Whether the pencils of n bands can be formed within ws_bytes
+bool gram_f64_i8_fits(int64_t N, int n, size_t ws_bytes) {
+    return gf_takes(n) && plan_gf(N, 2 * n, ws_bytes).bytes > 0 && plan_gf(N, 3 * n, ws_bytes).bytes > 0;
+}
+
+// Bytes of a workspace of its own that the pencils of up to n bands are to have, 0 where
+// `scratch` bytes that are free at that time do about as well or where n is not for this
+// form.  Only small bundles want one: the partial tiles of a wave of CTAs take 57 MB,
+// whatever the number of points (33 bands of 32^3 in the 9 MB of a bundle would take 12
+// times the stages).
+size_t gram_f64_i8_own_bytes(int64_t N, int n, size_t scratch) {
+    if (!gf_takes(n)) return 0;
+    const GfPlan two = plan_gf(N, 2 * n, GF_OWN_BYTES), three = plan_gf(N, 3 * n, GF_OWN_BYTES),
+                 have = plan_gf(N, 3 * n, scratch);
+    if (have.bytes > 0 && have.cost <= 1.1 * three.cost) return 0;
+    return std::max(two.bytes, three.bytes);
 }
 
 // A = scale U^T AU and B = scale U^T U (both m x m, full), m = nblk * n columns; *gave_up
@@ -467,8 +490,8 @@ size_t gram_f64_i8_bytes(int64_t N, int n) {
 qsb_status gram_f64_i8(int64_t N, int n, int nblk, const double* const* U, const double* const* AU, double scale,
                        double* A, double* B, void* ws, size_t ws_bytes, int* gave_up, cudaStream_t s) {
     const int p = n * nblk;
-    const GfPlan g = plan_gf(N, p);
-    if (ws_bytes < g.bytes) return fail(QSB_ERR_INVALID, "gram_f64_i8: workspace too small");
+    const GfPlan g = plan_gf(N, p, ws_bytes);
+    if (g.bytes == 0) return fail(QSB_ERR_INVALID, "gram_f64_i8: workspace too small");
     GfBundles b{};
     b.n = n;
     b.nblk = nblk;

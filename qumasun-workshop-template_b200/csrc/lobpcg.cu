@@ -334,7 +334,8 @@ struct qsb_eigensolver {
     double* vec = nullptr;           // small per-band vectors (eps, norms, scales): 8 x nmax
     double* partial = nullptr;       // reduction partials: nmax x nch
     double* gsmall = nullptr;        // tiles of the small real pencil (gram_small), few bands only
-    void* gi8 = nullptr;             // workspace of the large real pencil (gram_f64_i8), many bands only
+    void* gi8 = nullptr;             // workspace of the large real pencil (gram_f64_i8): TMP, or gi8_own
+    void* gi8_own = nullptr;         // where TMP is too small for it (few points)
     size_t gi8_bytes = 0;
     int nch = 0, chunk = 0;          // pieces of a band in the reductions, elements per piece
     void* swork = nullptr;
@@ -1372,13 +1373,6 @@ qsb_status qsb_eigensolver_create_ex(qsb_eigensolver** out, int64_t N, int n, in
     if (!es->mixed && !is_complex && gram_small_doubles(n) > 0 &&
         cudaMalloc((void**)&es->gsmall, gram_small_doubles(n) * sizeof(double)) != cudaSuccess)
         return cleanup(fail(QSB_ERR_NOMEM, "eigensolver: pencil tile allocation"));
-    if (!es->mixed && !is_complex && gram_f64_i8_bytes(N, n) > 0) {
-        es->gi8_bytes = gram_f64_i8_bytes(N, n);
-        if (cudaMalloc(&es->gi8, es->gi8_bytes) != cudaSuccess) {
-            cudaGetLastError();          // without it the blocks are DGEMMs
-            es->gi8 = nullptr;
-        }
-    }
     if (!es->mixed && is_complex) {
         const size_t mx = (size_t)3 * n;
         if (cudaMalloc((void**)&es->nxt, sizeof(double2) * (2 * mx * mx + (size_t)6 * n * n + 2 * mx * n)) !=
@@ -1403,6 +1397,23 @@ qsb_status qsb_eigensolver_create_ex(qsb_eigensolver** out, int64_t N, int n, in
     es->partial = es->vec + 8 * (size_t)n;
     if (cudaMalloc((void**)&es->info, 2 * sizeof(int)) != cudaSuccess)
         return cleanup(fail(QSB_ERR_NOMEM, "eigensolver: info allocation"));
+    if (!es->mixed && !is_complex) {
+        // TMP is not in use while a pencil is formed; where it is too small and there is no
+        // memory for another one either, the form runs in what TMP holds or (gram_f64_i8_fits)
+        // the pencil is formed by the library
+        const size_t tmp = es->L * n * sizeof(double), own = gram_f64_i8_own_bytes(N, n, tmp);
+        es->gi8 = es->TMP;
+        es->gi8_bytes = tmp;
+        if (own > 0) {
+            if (cudaMalloc(&es->gi8_own, own) == cudaSuccess) {
+                es->gi8 = es->gi8_own;
+                es->gi8_bytes = own;
+            } else {
+                cudaGetLastError();
+                es->gi8_own = nullptr;
+            }
+        }
+    }
     *out = es;
     return QSB_OK;
 }
@@ -1416,7 +1427,7 @@ qsb_status qsb_eigensolver_destroy(qsb_eigensolver* es) {
     for (float* p : b32)
         if (p) cudaFree(p);
     void* mw[11] = {es->su,   es->sau,  es->gpart, es->T2,     es->rc32, es->svq,
-                    es->rotw, es->rotc, es->nxt,   es->gsmall, es->gi8};
+                    es->rotw, es->rotc, es->nxt,   es->gsmall, es->gi8_own};
     for (void* p : mw)
         if (p) cudaFree(p);
     if (es->T) cudaFree(es->T);
@@ -1772,8 +1783,7 @@ qsb_status qsb_lobpcg_d(qsb_eigensolver* es, double dVol, int n, int iter_max, d
     }
     for (int k = 0; k < n; ++k) eigen_values[k] = eps[k];
 
-    const size_t gi8_need = es->gi8 ? gram_f64_i8_bytes(es->N, n) : 0;   // of these n bands
-    bool gi8 = gi8_need > 0 && gi8_need <= es->gi8_bytes;
+    bool gi8 = !es->gsmall && gram_f64_i8_fits(es->N, n, es->gi8_bytes);
     int iter;
     for (iter = 0; iter < iter_max; ++iter) {
         QSB_TRY(apply_op(es, n, es->R, es->AR, s));

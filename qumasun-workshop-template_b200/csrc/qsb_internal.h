@@ -197,12 +197,13 @@ size_t gram_small_doubles(int n);
 qsb_status gram_small(int64_t N, int n, int nblk, const double* const* U, const double* const* AU, double scale,
                       double* A, double* B, double* partial, cudaStream_t s);
 
-// The same of many bands on the INT8 tensor cores (gram_i8_f64.cu), in a workspace
-// of gram_f64_i8_bytes (0: n is not for this form).  From the first n that gram_small
+// The same of many bands on the INT8 tensor cores (gram_i8_f64.cu), in any workspace
+// that gram_f64_i8_fits.  From the first n that gram_small
 // does not take: faster than the 12 products at every size measured (33 to 200 bands,
-// 25^3 to 96^3 points; n = 33, 96^3: 3.4 -> 1.4 ms).
+// 25^3 to 96^3 points; n = 33, 96^3: 3.4 -> 1.9 ms).
 constexpr int GRAM_F64_I8_MIN_BANDS = 33;
-size_t gram_f64_i8_bytes(int64_t N, int n);
+bool gram_f64_i8_fits(int64_t N, int n, size_t ws_bytes);
+size_t gram_f64_i8_own_bytes(int64_t N, int n, size_t scratch);
 qsb_status gram_f64_i8(int64_t N, int n, int nblk, const double* const* U, const double* const* AU, double scale,
                        double* A, double* B, void* ws, size_t ws_bytes, int* gave_up, cudaStream_t s);
 
