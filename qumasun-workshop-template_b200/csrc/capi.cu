@@ -4,7 +4,12 @@
 #include <cmath>
 #include <cstring>
 #include <algorithm>
+#include <map>
+#include <mutex>
+#include <set>
 #include <string>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 namespace qsb {
@@ -37,6 +42,79 @@ int* device_error_word() {
         addr[dev] = (int*)p;
     }
     return addr[dev];
+}
+
+namespace {
+
+// Identity of the calling thread's current context (0: not to be had, nothing is
+// remembered then); a context made after a device reset has another one
+unsigned long long context_id() {
+    using Fn = int (*)(void*, unsigned long long*);          // cuCtxGetId
+    static const Fn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (Fn)p;
+    }();
+    unsigned long long id = 0;
+    if (!fn || fn(nullptr, &id) != 0) return 0;
+    return id + 1;
+}
+
+struct LaunchFacts {
+    std::mutex lock;
+    std::set<std::pair<const void*, unsigned long long>> allowed;
+    std::map<std::tuple<const void*, unsigned long long, int, size_t>, int> resident;
+};
+LaunchFacts& launch_facts() {
+    static LaunchFacts f;
+    return f;
+}
+
+}  // namespace
+
+qsb_status allow_shared_memory(const void* kernel) {
+    const unsigned long long ctx = context_id();
+    LaunchFacts& f = launch_facts();
+    if (ctx) {
+        std::lock_guard<std::mutex> g(f.lock);
+        if (f.allowed.count({kernel, ctx})) return QSB_OK;
+    }
+    int dev = 0, most = 0;
+    QSB_CUDA_TRY(cudaGetDevice(&dev));
+    QSB_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes a;
+    QSB_CUDA_TRY(cudaFuncGetAttributes(&a, kernel));
+    QSB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      most - (int)a.sharedSizeBytes));
+    if (ctx) {
+        std::lock_guard<std::mutex> g(f.lock);
+        f.allowed.insert({kernel, ctx});
+    }
+    return QSB_OK;
+}
+
+int resident_ctas(const void* kernel, int threads, size_t smem) {
+    const unsigned long long ctx = context_id();
+    const auto key = std::make_tuple(kernel, ctx, threads, smem);
+    LaunchFacts& f = launch_facts();
+    if (ctx) {
+        std::lock_guard<std::mutex> g(f.lock);
+        const auto it = f.resident.find(key);
+        if (it != f.resident.end()) return it->second;
+    }
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (ctx) {
+        std::lock_guard<std::mutex> g(f.lock);
+        f.resident.emplace(key, n);
+    }
+    return n;
 }
 
 static qsb_status check_grid(int nx, int ny, int nz) {

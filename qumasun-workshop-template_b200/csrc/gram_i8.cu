@@ -824,7 +824,7 @@ qsb_status gram_ozaki_tc(int64_t N, const void* A, int p, const void* B, int q, 
     }
     const int* ea = (const int*)(a + 4 * sa);
     const int* eb = (const int*)(b + 4 * sb);
-    QSB_CUDA_TRY(cudaFuncSetAttribute(gram_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OZ_SMEM));
+    QSB_TRY(allow_shared_memory(gram_i8_kernel));
     gram_i8_kernel<<<dim3(g.ntl, g.ksplit), OZ_THREADS, OZ_SMEM, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], g.kstages,
                                                                        g.ksplit, g.mtiles, upper ? 1 : 0,
                                                                        (double*)partial, device_error_word());
@@ -883,7 +883,7 @@ qsb_status ozaki_rotate(int64_t N, const void* Usplit, int K, const double* C, i
         if (!make_kmajor_map(&m[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a + k * sa, ldk, K, OZ_M, RT_KA) ||
             !make_kmajor_map(&m[4 + k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cs + k * cstride, kpad, q, RT_KB, RT_N))
             return fail(QSB_ERR_CUDA, "ozaki_rotate: tensor map encoding failed");
-    QSB_CUDA_TRY(cudaFuncSetAttribute(rot_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RT_SMEM));
+    QSB_TRY(allow_shared_memory(rot_i8_kernel));
     const int ntn = (q + RT_N - 1) / RT_N;
     const long long tiles = (long long)((N + OZ_M - 1) / OZ_M) * ntn;
     if (tiles > 0x7fffffffLL) return fail(QSB_ERR_INVALID, "ozaki_rotate: too many tiles");

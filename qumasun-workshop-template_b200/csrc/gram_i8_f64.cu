@@ -512,9 +512,9 @@ qsb_status gram_f64_i8(int64_t N, int n, int nblk, const double* const* U, const
     auto low = gram_f64_i8_kernel<8, 8, 4, 4>;
     auto mid = gram_f64_i8_kernel<4, 7, 0, 6>;
     auto top = gram_f64_i8_kernel<0, 3, 0, 3>;
-    QSB_CUDA_TRY(cudaFuncSetAttribute(low, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfLow::smem));
-    QSB_CUDA_TRY(cudaFuncSetAttribute(mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfMid::smem));
-    QSB_CUDA_TRY(cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GfTop::smem));
+    QSB_TRY(allow_shared_memory(low));
+    QSB_TRY(allow_shared_memory(mid));
+    QSB_TRY(allow_shared_memory(top));
     const int tiles = 2 * g.ntl;
     for (int c = 0; c < g.chunks; ++c) {
         const int64_t g0 = c * g.kc;

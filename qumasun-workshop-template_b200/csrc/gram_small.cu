@@ -142,7 +142,7 @@ qsb_status gram_small(int64_t N, int n, int nblk, const double* const* U, const 
     const int p = nblk * n, pt = (p + 7) / 8, tiles = pt * (pt + 1);
     const int ctas = (int)std::min<int64_t>(GS_CTAS, (N + GS_KC - 1) / GS_KC);
     const int smem = 2 * 8 * pt * GS_PITCH * (int)sizeof(double);
-    QSB_CUDA_TRY(cudaFuncSetAttribute(gram_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    QSB_TRY(allow_shared_memory(gram_small_kernel));
     gram_small_kernel<<<ctas, GS_WARPS * 32, smem, s>>>(b, n, p, pt, N, partial);
     gram_small_reduce_kernel<<<(tiles * 64 * 8 + 255) / 256, 256, 0, s>>>(partial, ctas, p, pt, scale, A, B);
     QSB_CUDA_TRY(cudaGetLastError());

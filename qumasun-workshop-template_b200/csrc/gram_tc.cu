@@ -392,7 +392,7 @@ qsb_status gram_split_tc(int64_t N, const void* A, int p, const void* B, int q, 
         !make_operand_map(&mbhi, b, ldk, q, GT_N) || !make_operand_map(&mblo, b + split_half_bytes(N, q), ldk, q, GT_N))
         return fail(QSB_ERR_CUDA, "gram_split_tc: tensor map encoding failed");
     auto kern = products == 4 ? gram_tc_kernel<4> : gram_tc_kernel<3>;
-    QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
+    QSB_TRY(allow_shared_memory(kern));
     kern<<<dim3(g.ntl, g.ksplit), GT_THREADS, GT_SMEM, s>>>(mahi, malo, mbhi, mblo, g.kstages, g.ksplit,
                                                                        g.mtiles, upper ? 1 : 0, (float*)partial,
                                                                        device_error_word());

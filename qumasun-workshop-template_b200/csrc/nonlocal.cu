@@ -801,7 +801,7 @@ qsb_status launch_proj(const NLDevice& d, const T* beta, int nb, const void* psi
                        double gy_dy, double gz_dz, double* partial, int ncol, cudaStream_t s) {
     using C = ProjCfg<T, CPLX, WM, CB>;
     auto kern = nl_proj_kernel<T, CPLX, WM, CB>;
-    QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    QSB_TRY(allow_shared_memory(kern));
     const dim3 grid((nb + CB - 1) / CB, d.n_chunks);
     kern<<<grid, PROJ_THREADS, C::SMEM, s>>>(d.chunk_order, d.chunk_begin, d.chunk_end, d.pt_idx, d.pt_xyz, beta,
                                              d.wmax, (const T*)psi, N, nb, gx_dx, gy_dy, gz_dz, partial, ncol);
@@ -840,7 +840,7 @@ qsb_status launch_proj_mma(const NLDevice& d, const ProjTables& tabs, const void
     auto kern = nl_proj_mma_kernel<T, CPLX, MT, NC, WARPS>;
     const MmaLayout ly((int)sizeof(T), NC, MT, tabs.n * d.wmax, CPLX);
     const int smem = std::max(WARPS * ly.warp_bytes, WARPS * 8 * MT * NC * 8);
-    QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    QSB_TRY(allow_shared_memory(kern));
     const dim3 grid((ncol + NC - 1) / NC, d.n_chunks);
     kern<<<grid, WARPS * 32, smem, s>>>(d.chunk_order, d.chunk_begin, d.chunk_end, d.pt_idx, d.pt_xyz, tabs,
                                             d.wmax, (const T*)psi, N, gx_dx, gy_dy, gz_dz, partial, table_stride,
@@ -1227,7 +1227,7 @@ qsb_status nl_apply(qsb_dtype dt, const NLDevice& d, int N, int nb, int is_compl
                             (size_t)2 * d.max_local * apply_row(d.wmax) * sizeof(double);                            \
         if (smem <= 200 * 1024) {                                                                                    \
             auto kern = d.wmax == W ? nl_apply_ring_kernel<T, C, W, true> : nl_apply_ring_kernel<T, C, W, false>;    \
-            QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));        \
+            QSB_TRY(allow_shared_memory(kern));        \
             kern<<<grid, APPLY_THREADS, smem, s>>>(d.cov_grid, d.n_cov, d.grid_ptr, d.ent_local, d.ent_xyz, B,       \
                                                    d.wmax, d.cta_ptr, d.cta_atoms, d.max_local, coef, ncol,          \
                                                    (T*)hpsi, (size_t)N, gx_dx, gy_dy, gz_dz);                        \

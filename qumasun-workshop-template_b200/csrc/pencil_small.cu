@@ -538,7 +538,7 @@ qsb_status pencil_small(int m, int n, bool cplx, double* Sa, double* Sb, double*
     auto kern = cplx ? (m <= 64 ? pencil_small_kernel<true, 2> : pencil_small_kernel<true, 3>)
                      : (m <= 64 ? pencil_small_kernel<false, 2> : pencil_small_kernel<false, 4>);
     if (cplx && m > 96) return fail(QSB_ERR_INVALID, "pencil_small: too many rows");   // past shared memory as well
-    QSB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    QSB_TRY(allow_shared_memory(kern));
     kern<<<1, PS_THREADS, smem, s>>>(m, n, Sa, Sb, W, info);
     QSB_CUDA_TRY(cudaGetLastError());
     return QSB_OK;

@@ -85,6 +85,19 @@ struct StencilLaunch {
     bool tma_ok = true;      // allow the TMA-pipelined kernel (else the register-prefetch one)
 };
 
+// Lets a kernel use as much dynamic shared memory as a CTA can have beside its
+// static part, once per kernel and context.  The limit is state of the function
+// that all host threads of a context share: set to the size of the launch at hand
+// it could shrink between another thread's call and its launch, which then fails.
+qsb_status allow_shared_memory(const void* kernel);
+template <typename... Args>
+qsb_status allow_shared_memory(void (*kernel)(Args...)) {
+    return allow_shared_memory((const void*)kernel);
+}
+// CTAs of `threads` threads and `smem` bytes of dynamic shared memory that fit an SM
+// (0: none), asked for once per kernel, context and shape
+int resident_ctas(const void* kernel, int threads, size_t smem);
+
 // Device-side error word (bit 0: a bounded wait in a kernel ran out), shared by
 // all kernels of the library; read and cleared with qsb_device_status().
 int* device_error_word();

@@ -1699,7 +1699,7 @@ bool launch_ws(const StencilLaunch& L, const FD8Coef& c, const KC<T>& k, cudaStr
                                          : fd8_ws_kernel<T, CPLX, MODE, CPLX, false, RY, S, true>)
                                   : (iso ? fd8_ws_kernel<T, CPLX, MODE, false, true, RY, S, true>
                                          : fd8_ws_kernel<T, CPLX, MODE, false, false, RY, S, true>);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (allow_shared_memory(kern) != QSB_OK) return false;
     kern<<<grid, block, C::SMEM, s>>>(m, (T*)L.out, L.nx, L.ny, L.nz, zchunk, tiles, nzc, (int)items, k,
                                       device_error_word(), compute_poll_limit());
     return true;
@@ -1747,15 +1747,9 @@ bool launch_wq(const StencilLaunch& L, const FD8Coef& c, const KC<float>& k, int
     const bool grad = CPLX && c.has_grad;
     auto kern = grad ? fd8_wq_kernel<CPLX, MODE, CPLX, A> : fd8_wq_kernel<CPLX, MODE, false, A>;
     const int threads = (A * b + 1) * 32;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ly.total) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, ly.total) != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        return false;
-    }
+    if (allow_shared_memory(kern) != QSB_OK) return false;
+    const int per_sm = resident_ctas((const void*)kern, threads, ly.total);
+    if (per_sm < 1) return false;
     // z chunks: each costs the 8 planes of its halo again, and the last wave of
     // CTAs is rarely full: the split with the smallest waves x planes
     const long long tiles = (long long)((L.nx + TXQ - 1) / TXQ) * ((L.ny + TY - 1) / TY);
@@ -1814,12 +1808,12 @@ bool launch_zacc(const StencilLaunch& L, const FD8Coef& c, const KC<T>& k, cudaS
         return false;
     if (CPLX && c.has_grad) {
         auto kern = fd8_zacc_kernel<T, CPLX, MODE, CPLX, ZY, RY, S, MINB>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        if (allow_shared_memory(kern) != QSB_OK) return false;
         kern<<<grid, block, C::SMEM, s>>>(map, (T*)L.out, (const T*)L.in, (const T*)L.V, L.nx, L.ny, L.nz, zchunk, k,
                                           device_error_word());
     } else {
         auto kern = fd8_zacc_kernel<T, CPLX, MODE, false, ZY, RY, S, MINB>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        if (allow_shared_memory(kern) != QSB_OK) return false;
         kern<<<grid, block, C::SMEM, s>>>(map, (T*)L.out, (const T*)L.in, (const T*)L.V, L.nx, L.ny, L.nz, zchunk, k,
                                           device_error_word());
     }
