@@ -1588,16 +1588,14 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const EncodeTiledFn fn = [] {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    }
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (EncodeTiledFn)p;
+    }();
     return fn;
 }
 
@@ -1622,14 +1620,12 @@ bool make_plane_map(CUtensorMap* map, const void* base, int nx, int ny, long lon
 // prefetch, no TMA), 3 fd8_zacc_kernel; QSB_STENCIL=ws|reg|zacc overrides it for
 // A/B timing.
 int stencil_variant() {
-    static int v = -1;
-    if (v < 0) {
+    static const int v = [] {
         const char* e = std::getenv("QSB_STENCIL");
-        v = 0;
-        if (e && std::string(e) == "reg") v = 2;
-        if (e && std::string(e) == "zacc") v = 3;
-
-    }
+        if (e && std::string(e) == "reg") return 2;
+        if (e && std::string(e) == "zacc") return 3;
+        return 0;
+    }();
     return v;
 }
 

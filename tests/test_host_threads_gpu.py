@@ -79,3 +79,44 @@ def test_no_call_disturbs_another_thread(qsb, what):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+FIRST = r"""
+import threading
+import torch
+import qsb
+n, nb, h = 32, 4, 0.3
+N = n ** 3
+psi = torch.rand(nb, N, dtype=torch.float64, device="cuda") - 0.5
+V = torch.rand(N, dtype=torch.float64, device="cuda")
+hams = []
+for _ in range(8):
+    H = qsb.Hamiltonian(n, n, n, h, h, h)
+    H.set_potential(V)
+    hams.append(H)
+outs = [torch.empty_like(psi) for _ in hams]
+torch.cuda.synchronize()
+start = threading.Barrier(8)
+def work(k):
+    start.wait()
+    hams[k].apply(psi, outs[k])
+threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+torch.cuda.synchronize()
+print(all(torch.equal(o, outs[0]) for o in outs))
+"""
+
+
+def test_first_calls_of_a_process_from_several_threads(qsb):
+    """Every thread's first stencil finds the tensor-map encoder, whoever looked it up:
+    without it a thread would take another kernel, with another rounding."""
+    import os
+    import subprocess
+    import sys
+    pkg = os.path.dirname(os.path.abspath(qsb.__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([pkg, os.environ.get("PYTHONPATH", "")]))
+    for _ in range(3):
+        r = subprocess.run([sys.executable, "-c", FIRST], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        assert r.stdout.strip().splitlines()[-1] == "True"
