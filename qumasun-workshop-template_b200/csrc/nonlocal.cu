@@ -41,15 +41,64 @@ void dfree(T*& p) {
     p = nullptr;
 }
 
-template <typename T>
-qsb_status dupload(T*& dst, const T* src, size_t n) {
-    dfree(dst);
-    if (n == 0) return QSB_OK;
-    cudaError_t e = cudaMalloc((void**)&dst, n * sizeof(T));
-    if (e != cudaSuccess) { dst = nullptr; return fail(QSB_ERR_NOMEM, "nonlocal tables: cudaMalloc failed"); }
-    QSB_CUDA_TRY(cudaMemcpy(dst, src, n * sizeof(T), cudaMemcpyHostToDevice));
-    return QSB_OK;
-}
+// Device copies of host tables in two allocations, the short ones of each going up in
+// one copy, so that a small cell's two dozen tables do not cost as many allocations
+// and waits (10.5 -> 10.2 ms for two atoms on 32^3, 12.9 -> 12.2 for three on 45 x 50 x 63).
+// Tables of a few KB stay apart from the large ones: the allocator serves what they
+// take, and the workspace of the first apply after them, from one small block (in
+// one allocation with the rest that workspace cost the first apply 0.5 ms).
+class TableUpload {
+public:
+    template <typename T>
+    void add(T*& dst, const T* src, size_t n) {
+        dst = nullptr;
+        if (n > 0) items_.push_back({&dst, src, n * sizeof(T), 0});
+    }
+    template <typename T>
+    void add(T*& dst, const std::vector<T>& v) {
+        add(dst, v.data(), v.size());
+    }
+    // base: the allocations (also those made before an error), null where nothing is needed
+    qsb_status run(void* (&base)[2]) {
+        std::stable_sort(items_.begin(), items_.end(), [](const Item& a, const Item& b) { return a.bytes < b.bytes; });
+        const auto cut = std::find_if(items_.begin(), items_.end(), [](const Item& it) { return it.bytes > TINY; });
+        QSB_TRY(place(items_.begin(), cut, base[0]));
+        return place(cut, items_.end(), base[1]);
+    }
+
+private:
+    static constexpr size_t TINY = (size_t)1 << 16, SHORT = (size_t)1 << 20;
+    struct Item {
+        void* dst;                 // the pointer to set
+        const void* src;
+        size_t bytes, off;
+    };
+    using Iter = std::vector<Item>::iterator;
+    static qsb_status place(Iter first, Iter last, void*& base) {
+        size_t total = 0, packed = 0;
+        for (Iter it = first; it != last; ++it) {
+            it->off = total;
+            total += (it->bytes + 255) / 256 * 256;
+            if (it->bytes <= SHORT) packed = total;
+        }
+        if (total == 0) return QSB_OK;
+        if (cudaMalloc(&base, total) != cudaSuccess) {
+            cudaGetLastError();
+            base = nullptr;
+            return fail(QSB_ERR_NOMEM, "nonlocal tables: cudaMalloc failed");
+        }
+        std::vector<unsigned char> stage(packed);
+        for (Iter it = first; it != last; ++it) {
+            void* const at = (unsigned char*)base + it->off;
+            if (it->bytes <= SHORT) std::memcpy(stage.data() + it->off, it->src, it->bytes);
+            else QSB_CUDA_TRY(cudaMemcpy(at, it->src, it->bytes, cudaMemcpyHostToDevice));
+            std::memcpy(it->dst, &at, sizeof(at));      // whatever type of pointer it is
+        }
+        if (packed > 0) QSB_CUDA_TRY(cudaMemcpy(base, stage.data(), packed, cudaMemcpyHostToDevice));
+        return QSB_OK;
+    }
+    std::vector<Item> items_;
+};
 
 inline int fold(int v, int n) {
     int m = v % n;
@@ -920,12 +969,16 @@ __global__ void nl_energy_force_kernel(const double* __restrict__ c, const doubl
 }  // namespace
 
 void nl_free(NLDevice& d) {
-    dfree(d.pt_idx); dfree(d.pt_xyz); dfree(d.pt_beta64); dfree(d.pt_beta32);
-    dfree(d.atom_width); dfree(d.atom_proj_off); dfree(d.atom_E);
-    dfree(d.chunk_atom); dfree(d.chunk_begin); dfree(d.chunk_end); dfree(d.chunk_order);
-    dfree(d.atom_chunk_begin); dfree(d.atom_chunk_end);
-    dfree(d.grid_ptr); dfree(d.cov_grid); dfree(d.ent_atom); dfree(d.ent_local); dfree(d.cta_ptr); dfree(d.cta_atoms); dfree(d.ent_xyz);
-    dfree(d.ent_beta64); dfree(d.ent_beta32);
+    for (void*& p : d.tables) dfree(p);
+    d.pt_idx = d.pt_xyz = nullptr;
+    d.pt_beta64 = nullptr;
+    d.pt_beta32 = nullptr;
+    d.atom_width = d.atom_proj_off = nullptr;
+    d.atom_E = nullptr;
+    d.chunk_atom = d.chunk_order = d.chunk_begin = d.chunk_end = d.atom_chunk_begin = d.atom_chunk_end = nullptr;
+    d.grid_ptr = d.cov_grid = d.ent_atom = d.ent_local = d.cta_ptr = d.cta_atoms = d.ent_xyz = nullptr;
+    d.ent_beta64 = nullptr;
+    d.ent_beta32 = nullptr;
     dfree(d.pt_dbeta64); dfree(d.pt_dbeta32);
     d.n_atoms = 0; d.wmax = 0; d.n_points = 0; d.total_proj = 0; d.n_chunks = 0; d.n_cov = 0; d.max_local = 0;
     d.h_atom_width.clear(); d.h_atom_proj_off.clear(); d.h_npts.clear(); d.h_src.clear();
@@ -1057,29 +1110,32 @@ qsb_status nl_upload(NLDevice& d, int nx, int ny, int nz, int n_atoms, const int
     }
 
     std::vector<float> b32(b64.begin(), b64.end()), e_b32(e_b64.begin(), e_b64.end());
-    QSB_TRY(dupload(d.pt_idx, idx.data(), idx.size()));
-    QSB_TRY(dupload(d.pt_xyz, xyz.data(), xyz.size()));
-    QSB_TRY(dupload(d.pt_beta64, b64.data(), b64.size()));
-    QSB_TRY(dupload(d.pt_beta32, b32.data(), b32.size()));
-    QSB_TRY(dupload(d.atom_width, widths, (size_t)n_atoms));
-    QSB_TRY(dupload(d.atom_proj_off, d.h_atom_proj_off.data(), (size_t)n_atoms));
-    QSB_TRY(dupload(d.atom_E, E.data(), E.size()));
-    QSB_TRY(dupload(d.chunk_atom, chunk_atom.data(), chunk_atom.size()));
-    QSB_TRY(dupload(d.chunk_order, corder.data(), corder.size()));
-    QSB_TRY(dupload(d.chunk_begin, chunk_b.data(), chunk_b.size()));
-    QSB_TRY(dupload(d.chunk_end, chunk_e.data(), chunk_e.size()));
-    QSB_TRY(dupload(d.atom_chunk_begin, acb.data(), acb.size()));
-    QSB_TRY(dupload(d.atom_chunk_end, ace.data(), ace.size()));
-    QSB_TRY(dupload(d.grid_ptr, gptr.data(), gptr.size()));
-    QSB_TRY(dupload(d.cov_grid, cov.data(), cov.size()));
-    QSB_TRY(dupload(d.ent_atom, e_atom.data(), e_atom.size()));
-    QSB_TRY(dupload(d.ent_local, e_local.data(), e_local.size()));
-    QSB_TRY(dupload(d.cta_ptr, cptr.data(), cptr.size()));
-    QSB_TRY(dupload(d.cta_atoms, catoms.data(), catoms.size()));
-    QSB_TRY(dupload(d.ent_xyz, e_xyz.data(), e_xyz.size()));
-    QSB_TRY(dupload(d.ent_beta64, e_b64.data(), e_b64.size()));
-    QSB_TRY(dupload(d.ent_beta32, e_b32.data(), e_b32.size()));
-    return QSB_OK;
+    TableUpload up;
+    up.add(d.pt_idx, idx);
+    up.add(d.pt_xyz, xyz);
+    up.add(d.pt_beta64, b64);
+    up.add(d.pt_beta32, b32);
+    up.add(d.atom_width, widths, (size_t)n_atoms);
+    up.add(d.atom_proj_off, d.h_atom_proj_off.data(), (size_t)n_atoms);
+    up.add(d.atom_E, E);
+    up.add(d.chunk_atom, chunk_atom);
+    up.add(d.chunk_order, corder);
+    up.add(d.chunk_begin, chunk_b);
+    up.add(d.chunk_end, chunk_e);
+    up.add(d.atom_chunk_begin, acb);
+    up.add(d.atom_chunk_end, ace);
+    up.add(d.grid_ptr, gptr);
+    up.add(d.cov_grid, cov);
+    up.add(d.ent_atom, e_atom);
+    up.add(d.ent_local, e_local);
+    up.add(d.cta_ptr, cptr);
+    up.add(d.cta_atoms, catoms);
+    up.add(d.ent_xyz, e_xyz);
+    up.add(d.ent_beta64, e_b64);
+    up.add(d.ent_beta32, e_b32);
+    const qsb_status st = up.run(d.tables);
+    if (st != QSB_OK) nl_free(d);           // no projectors rather than half of them
+    return st;
 }
 
 size_t nl_workspace_bytes(const NLDevice& d, int ncol) {

@@ -130,6 +130,7 @@ struct NLDevice {
     int n_atoms = 0;
     int wmax = 0;                  // max projectors per atom (tables padded to wmax)
     int64_t n_points = 0;          // total points over atoms
+    void* tables[2] = {nullptr, nullptr};   // allocations that hold all tables but the gradients
     int total_proj = 0;            // sum of widths
     // atom-major point arrays
     int* pt_idx = nullptr;         // folded grid index
