@@ -73,6 +73,15 @@ __device__ __forceinline__ int wrap_up(int v, int n) {
     return v < n ? v : v % n;
 }
 
+// Weighted sum of the neighbours at distance 4, 3, 2, 1 in FP32, w[i] the weight of
+// distance i + 1: the order of roundings of every FP32 stencil (sum4x along x)
+__device__ __forceinline__ float sum4(const float (&w)[4], float a4, float a3, float a2, float a1) {
+    return __fmaf_rn(w[0], a1, __fmaf_rn(w[1], a2, __fmaf_rn(w[3], a4, __fmul_rn(w[2], a3))));
+}
+__device__ __forceinline__ float sum4x(const float (&w)[4], float a4, float a3, float a2, float a1) {
+    return __fmaf_rn(w[0], a1, __fmaf_rn(w[1], a2, __fmaf_rn(w[2], a3, __fmul_rn(w[3], a4))));
+}
+
 // One CTA: a TX x TY tile (TY = BY*RY) of one band (both SoA planes for
 // complex), marching z over [z0, z1).  Thread (tx, ty) owns the RY
 // consecutive grid rows y0 + ty*RY + i at x0 + tx and keeps their z columns
@@ -239,23 +248,42 @@ __device__ __forceinline__ void fd8_tile(const T* __restrict__ in, T* __restrict
 #define QZ(k) q[c][i][(p + (k)) % 9]
                         const T xm4 = s[sy][sx - 4], xm3 = s[sy][sx - 3], xm2 = s[sy][sx - 2], xm1 = s[sy][sx - 1];
                         const T xp1 = s[sy][sx + 1], xp2 = s[sy][sx + 2], xp3 = s[sy][sx + 3], xp4 = s[sy][sx + 4];
-                        T d = k.c0 * QZ(4);
-                        d += k.cx[3] * (xp4 + xm4) + k.cx[2] * (xp3 + xm3) + k.cx[1] * (xp2 + xm2) +
-                             k.cx[0] * (xp1 + xm1);
-                        d += k.cy[3] * (col[i + 8] + col[i]) + k.cy[2] * (col[i + 7] + col[i + 1]) +
-                             k.cy[1] * (col[i + 6] + col[i + 2]) + k.cy[0] * (col[i + 5] + col[i + 3]);
-                        d += k.cz[3] * (QZ(8) + QZ(0)) + k.cz[2] * (QZ(7) + QZ(1)) + k.cz[1] * (QZ(6) + QZ(2)) +
-                             k.cz[0] * (QZ(5) + QZ(3));
-                        if constexpr (sizeof(T) == 4) d = fmaf(k.c0lo, QZ(4), d);
-                        res[c][i] = d;
-                        if (GRAD) {
-                            T g = k.ax[3] * (xp4 - xm4) + k.ax[2] * (xp3 - xm3) + k.ax[1] * (xp2 - xm2) +
-                                  k.ax[0] * (xp1 - xm1);
-                            g += k.ay[3] * (col[i + 8] - col[i]) + k.ay[2] * (col[i + 7] - col[i + 1]) +
-                                 k.ay[1] * (col[i + 6] - col[i + 2]) + k.ay[0] * (col[i + 5] - col[i + 3]);
-                            g += k.az[3] * (QZ(8) - QZ(0)) + k.az[2] * (QZ(7) - QZ(1)) + k.az[1] * (QZ(6) - QZ(2)) +
-                                 k.az[0] * (QZ(5) - QZ(3));
-                            grd[c][i] = g;
+                        if constexpr (sizeof(T) == 4) {
+                            // one order of roundings for every FP32 kernel (here, in the batched launch and
+                            // in fd8_wq_kernel), written out: left to the compiler, the contractions of
+                            // this code differed between two kernels it was compiled into
+                            const float xs = sum4x(k.cx, xp4 + xm4, xp3 + xm3, xp2 + xm2, xp1 + xm1);
+                            const float ys = sum4(k.cy, col[i + 8] + col[i], col[i + 7] + col[i + 1],
+                                                  col[i + 6] + col[i + 2], col[i + 5] + col[i + 3]);
+                            const float zs = sum4(k.cz, QZ(8) + QZ(0), QZ(7) + QZ(1), QZ(6) + QZ(2), QZ(5) + QZ(3));
+                            const float d = __fadd_rn(__fadd_rn(__fmaf_rn(k.c0, QZ(4), xs), ys), zs);
+                            res[c][i] = __fmaf_rn(k.c0lo, QZ(4), d);
+                            if (GRAD) {
+                                const float gx = sum4x(k.ax, xp4 - xm4, xp3 - xm3, xp2 - xm2, xp1 - xm1);
+                                const float gy = sum4(k.ay, col[i + 8] - col[i], col[i + 7] - col[i + 1],
+                                                      col[i + 6] - col[i + 2], col[i + 5] - col[i + 3]);
+                                const float gz = sum4(k.az, QZ(8) - QZ(0), QZ(7) - QZ(1), QZ(6) - QZ(2),
+                                                      QZ(5) - QZ(3));
+                                grd[c][i] = __fadd_rn(__fadd_rn(gx, gy), gz);
+                            }
+                        } else {
+                            T d = k.c0 * QZ(4);
+                            d += k.cx[3] * (xp4 + xm4) + k.cx[2] * (xp3 + xm3) + k.cx[1] * (xp2 + xm2) +
+                                 k.cx[0] * (xp1 + xm1);
+                            d += k.cy[3] * (col[i + 8] + col[i]) + k.cy[2] * (col[i + 7] + col[i + 1]) +
+                                 k.cy[1] * (col[i + 6] + col[i + 2]) + k.cy[0] * (col[i + 5] + col[i + 3]);
+                            d += k.cz[3] * (QZ(8) + QZ(0)) + k.cz[2] * (QZ(7) + QZ(1)) + k.cz[1] * (QZ(6) + QZ(2)) +
+                                 k.cz[0] * (QZ(5) + QZ(3));
+                            res[c][i] = d;
+                            if (GRAD) {
+                                T g = k.ax[3] * (xp4 - xm4) + k.ax[2] * (xp3 - xm3) + k.ax[1] * (xp2 - xm2) +
+                                      k.ax[0] * (xp1 - xm1);
+                                g += k.ay[3] * (col[i + 8] - col[i]) + k.ay[2] * (col[i + 7] - col[i + 1]) +
+                                     k.ay[1] * (col[i + 6] - col[i + 2]) + k.ay[0] * (col[i + 5] - col[i + 3]);
+                                g += k.az[3] * (QZ(8) - QZ(0)) + k.az[2] * (QZ(7) - QZ(1)) + k.az[1] * (QZ(6) - QZ(2)) +
+                                     k.az[0] * (QZ(5) - QZ(3));
+                                grd[c][i] = g;
+                            }
                         }
 #undef QZ
                     }
@@ -276,8 +304,13 @@ __device__ __forceinline__ void fd8_tile(const T* __restrict__ in, T* __restrict
                         if (CPLX) dst[NC - 1][gidx] = ep[p % 3][NE - 1][i] + r1;
                     } else {
                         const T v = ep[p % 3][0][i];
-                        dst[0][gidx] = v * q[0][i][(p + 4) % 9] + r0;
-                        if (CPLX) dst[NC - 1][gidx] = v * q[NC - 1][i][(p + 4) % 9] + r1;
+                        if constexpr (sizeof(T) == 4) {
+                            dst[0][gidx] = __fmaf_rn(v, q[0][i][(p + 4) % 9], r0);
+                            if (CPLX) dst[NC - 1][gidx] = __fmaf_rn(v, q[NC - 1][i][(p + 4) % 9], r1);
+                        } else {
+                            dst[0][gidx] = v * q[0][i][(p + 4) % 9] + r0;
+                            if (CPLX) dst[NC - 1][gidx] = v * q[NC - 1][i][(p + 4) % 9] + r1;
+                        }
                     }
                 }
             }
@@ -1520,7 +1553,7 @@ fd8_wq_kernel(const __grid_constant__ WsMaps maps, float* __restrict__ out, int 
                             const f32x2 x4 = add2(ap[4 + h], ap[h]), x2 = add2(ap[3 + h], ap[1 + h]);
                             const f32x2 x3 = pk(at(o + 3) + at(o - 3), at(o + 4) + at(o - 2));
                             const f32x2 x1 = pk(at(o + 1) + at(o - 1), at(o + 2) + at(o));
-                            // the products in fd8_kernel's contraction order, so that the two agree bit for bit
+                            // sum4x() and sum4() on pairs, fd8_tile's order: the same bits
                             f32x2 xs = fma2(k.cx[2], x3, mul2(k.cx[3], x4));
                             xs = fma2(k.cx[1], x2, xs);
                             xs = fma2(k.cx[0], x1, xs);
@@ -1618,7 +1651,7 @@ bool make_plane_map(CUtensorMap* map, const void* base, int nx, int ny, long lon
 // Stencil kernel choice (FP64): 0 fd8_ws_kernel (default; fd8_zacc_kernel where its tiling
 // does not apply, fd8_kernel without 16-byte alignment), 2 fd8_kernel (register
 // prefetch, no TMA), 3 fd8_zacc_kernel; QSB_STENCIL=ws|reg|zacc overrides it for
-// A/B timing.
+// A/B timing.  FP32 takes fd8_wq_kernel at 0 where a tiling fits, else fd8_kernel.
 int stencil_variant() {
     static const int v = [] {
         const char* e = std::getenv("QSB_STENCIL");
@@ -1896,8 +1929,8 @@ qsb_status launch_dtype(const StencilLaunch& L, const FD8Coef& c, cudaStream_t s
 // outputs, the register-prefetch kernel -- two runs each after a warm one, on
 // the caller's stream with CUDA events, keeps the fastest for that shape, and
 // runs it once more so the output is its own.  Decisions are logged
-// (qsb_autotune_report).  FP32 keeps the register-prefetch kernel (its summation
-// order), MODE 0 ("+=") the default order of kernels.
+// (qsb_autotune_report).  FP32 keeps the default (fd8_wq_kernel, or fd8_kernel where no
+// tiling fits: one summation order), MODE 0 ("+=") the default order of kernels.
 struct TuneState {
     std::mutex mu;
     bool on = false;

@@ -83,3 +83,27 @@ def test_autotuned_applies_equal_untuned_and_are_logged(qsb):
         assert f"stencil {n}x{n}x{n} real" in log, log
     assert "ham_apply_batch 3 systems" in log and "->" in log, log
     assert qsb.device_status() == 0
+
+
+def test_f32_batch_equals_per_system_apply_bit_for_bit(qsb):
+    """The persistent launch's tiles, the TMA-fed stencil of the larger systems and the
+    per-system kernels sum in one order: systems on both sides of the line that
+    separates them, and one without a 16-byte row pitch."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    hams, psis = [], []
+    for nx, ny, nz, nb, na in [(32, 32, 32, 3, 1), (64, 64, 64, 24, 2), (40, 48, 56, 9, 0), (33, 20, 18, 5, 1),
+                               (56, 32, 40, 40, 3)]:
+        rng = np.random.default_rng(nx)
+        H = qsb.Hamiltonian(nx, ny, nz, 0.25, 0.25, 0.25)
+        H.set_potential(torch.rand(nx * ny * nz, dtype=torch.float64, device="cuda", generator=gen) - 0.5)
+        if na:
+            H.set_gth_projectors(rng.uniform(0, 4, (na, 3)), [0] * na, [O.GTH_BCC["nl"]], [O.GTH_BCC["r"]],
+                                 [O.GTH_BCC["h"]], O.RCUT_FACTOR)
+        hams.append(H)
+        psis.append(torch.rand(nb, nx * ny * nz, dtype=torch.float32, device="cuda", generator=gen) - 0.5)
+    got = [torch.empty_like(p) for p in psis]
+    qsb.apply_batch(hams, psis, got)
+    for H, p, g in zip(hams, psis, got):
+        assert torch.equal(H.apply(p, torch.empty_like(p)).view(torch.int32), g.view(torch.int32))
+    assert qsb.device_status() == 0

@@ -46,3 +46,51 @@ def test_f32_stencil_equals_f64(qsb, grid, cplx):
         assert np.linalg.norm(e) / np.sqrt(e.size) < 2e-6 * rms
         assert np.max(np.abs(e)) < 2e-5 * rms
     assert qsb.device_status() == 0
+
+
+# every form of both kernels: (complex, Bloch vector), += and V psi + forms, on grids with edge
+# tiles, z chunks and odd band counts
+SAME_BITS = r"""
+import sys
+import torch
+import qsb
+out = []
+for nx, ny, nz, nb in [(32, 16, 4, 3), (48, 16, 8, 1), (36, 20, 5, 2), (64, 48, 33, 5), (100, 36, 12, 3), (52, 84, 40, 2),
+                       (96, 96, 20, 7)]:
+    N, d = nx * ny * nz, (0.2, 0.25, 0.21)
+    gen = torch.Generator(device="cuda").manual_seed(nx + 7 * ny)
+    V = torch.rand(N, dtype=torch.float64, device="cuda", generator=gen) - 0.5
+    H = qsb.Hamiltonian(nx, ny, nz, *d)
+    H.set_potential(V)
+    for cplx, g in [(False, (0.0, 0.0, 0.0)), (True, (0.0, 0.0, 0.0)), (True, (0.1, -0.2, 0.3))]:
+        p = torch.rand((nb, 2, N) if cplx else (nb, N), dtype=torch.float32, device="cuda", generator=gen) - 0.5
+        a = torch.rand(p.shape, dtype=torch.float32, device="cuda", generator=gen)
+        if cplx:
+            qsb.laplacian_kpoint8th(a, p, -0.5, *d, g, (nx, ny, nz))
+        else:
+            qsb.laplacian8th(a, p, -0.5, *d, (nx, ny, nz))
+        h = torch.empty_like(p)
+        H.apply(p, h, is_complex=cplx, g=g)
+        out += [a.cpu(), h.cpu()]
+torch.save(out, sys.argv[1])
+"""
+
+
+def test_f32_stencil_equals_the_register_kernel_bit_for_bit(qsb, tmp_path):
+    """fd8_wq_kernel against fd8_kernel (QSB_STENCIL=reg in a child process): the
+    same FP32 contractions in the same order, whatever kernel a grid takes."""
+    import os
+    import subprocess
+    import sys
+    import torch
+    pkg = os.path.dirname(os.path.abspath(qsb.__file__))
+    res = []
+    for variant in ("ws", "reg"):
+        path = str(tmp_path / (variant + ".pt"))
+        env = dict(os.environ, QSB_STENCIL=variant, PYTHONPATH=os.pathsep.join([pkg, os.environ.get("PYTHONPATH", "")]))
+        r = subprocess.run([sys.executable, "-c", SAME_BITS, path], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        res.append(torch.load(path))
+    assert len(res[0]) == len(res[1]) == 42
+    for a, b in zip(*res):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
