@@ -27,7 +27,7 @@ constexpr int FFT_CHUNK = 32;     // most bands per batched transform
 // pass of the two transforms, the pack, the multiplier and the finish: chunks
 // whose spectra stay in the 126 MB L2 between the passes leave DRAM the psi
 // reads and H psi writes (at 32 bands, 226 MB of spectra at 96^3, every pass went
-// to DRAM).  A quarter of L2 beside the passes' psi and H psi.
+// to DRAM).  About half of L2; the passes' psi and H psi go through the rest.
 constexpr size_t FFT_L2_BYTES = 60u << 20;
 inline int fields_per_chunk(size_t field_bytes, int most) {
     const size_t n = FFT_L2_BYTES / std::max<size_t>(1, field_bytes);

@@ -81,20 +81,72 @@ def test_ritz_values_and_orthonormal_bands(qsb, cplx, n, flat):
     assert np.allclose(np.sort(ev), ref, rtol=1e-10, atol=1e-10)
 
 
-def test_indefinite_overlap_takes_the_overlap_basis(qsb):
-    """Two equal bands make the overlap singular: the step is solved on the rest."""
+def _cell(qsb, n, V, h=0.4, m=16):
     import torch
-    m, h, n = 16, 0.4, 6
-    N, dV = m ** 3, h ** 3
-    gen = torch.Generator(device="cuda").manual_seed(1)
     H = qsb.Hamiltonian(m, m, m, h, h, h)
-    H.set_potential(torch.rand(N, dtype=torch.float64, device="cuda", generator=gen))
-    X = torch.rand(n, N, dtype=torch.float64, device="cuda", generator=gen) - 0.5
-    qsb.orthonormalize(X, N, dV)
-    X[3] = X[2]
-    es = qsb.EigenSolver(N, n, False, "fp64")
+    H.set_potential(V)
+    es = qsb.EigenSolver(m ** 3, n, False, "fp64")
     es.set_hamiltonian(H)
+    return H, es
+
+
+def _bands(qsb, n, dV, m=16):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    V = torch.rand(m ** 3, dtype=torch.float64, device="cuda", generator=gen)
+    X = torch.rand(n, m ** 3, dtype=torch.float64, device="cuda", generator=gen) - 0.5
+    qsb.orthonormalize(X, m ** 3, dV)
+    return V, X
+
+
+def test_equal_bands_stay_defined(qsb):
+    """Two equal bands make the overlap singular: whichever way its pivots round, the
+    steps are solved and the bands stay finite."""
+    import torch
+    n, dV = 6, 0.4 ** 3
+    V, X = _bands(qsb, n, dV)
+    X[3] = X[2]
+    H, es = _cell(qsb, n, V)
     ev = np.zeros(n)
     es.lobpcg_d(dV, n, 2, ev, X, torch.zeros_like(X), True)
     chol, basis = es.solve_stats()
     assert chol + basis == 2 and np.all(np.isfinite(ev)) and bool(torch.isfinite(X).all())
+
+
+def test_indefinite_overlap_takes_the_overlap_basis(qsb):
+    """Kept directions of zero make the overlap's last pivots zero, exactly: the step is
+    solved on the rest of the basis, whose Ritz values numpy gives."""
+    import torch
+    n, dV = 6, 0.4 ** 3
+    V, X = _bands(qsb, n, dV)
+    H, es = _cell(qsb, n, V)
+    apply = lambda Z: H.apply(Z.contiguous(), torch.empty_like(Z))
+    AX = apply(X)
+    R = AX - (X * AX).sum(1, keepdim=True) * dV * X
+    U = torch.cat([X, R / torch.linalg.norm(R, dim=1, keepdim=True)])
+    A, S = (U @ apply(U).T).cpu().numpy(), (U @ U.T).cpu().numpy()
+    L = np.linalg.cholesky(S)
+    T = np.linalg.solve(L, np.linalg.solve(L, 0.5 * (A + A.T)).T)
+    ref = np.linalg.eigvalsh(0.5 * (T + T.T))[:n]
+    ev = np.zeros(n)
+    es.lobpcg_d(dV, n, 1, ev, X, torch.zeros_like(X), False)
+    assert es.solve_stats() == (0, 1)
+    assert np.abs(np.sort(ev) - ref).max() < 1e-10 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n", [2, 12])
+def test_unresolved_vectors_take_the_library(qsb, n):
+    """An operator of 2^-470 (lengths of 2^235): the inverse iteration's squares overflow,
+    the one-launch solve reports vectors it cannot make orthonormal, and the library's
+    solution of the same pencil comes back: the Ritz values of the unscaled operator."""
+    import torch
+    V, X0 = _bands(qsb, n, 1.0)
+    out = []
+    for s in (0, 235):
+        H, es = _cell(qsb, n, V * 2.0 ** (-2 * s), h=2.0 ** s * 0.4)
+        X, ev = X0.clone(), np.zeros(n)
+        es.lobpcg_d(1.0, n, 1, ev, X, torch.zeros_like(X), True)
+        assert es.solve_stats() == (1, 0)
+        assert float((X @ X.T - torch.eye(n, dtype=torch.float64, device="cuda")).abs().max()) < 1e-10
+        out.append(np.sort(ev) * 2.0 ** (2 * s))
+    assert np.abs(out[0] - out[1]).max() < 1e-10 * np.abs(out[0]).max()
