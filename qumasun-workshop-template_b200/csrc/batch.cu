@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -49,6 +50,12 @@ extern "C" qsb_status qsb_ham_apply_batch(qsb_dtype dtype, int n_sys, qsb_ham* c
         if (hams[i]->kinetic != 0)
             return qsb::fail(QSB_ERR_INVALID, "ham_apply_batch: the batched stencil is the FD8 kinetic (system " +
                                                   std::to_string(i) + " is set to FFT)");
+    }
+    // an operator listed twice has one workspace for its coefficients: one apply after the other
+    if (std::set<const qsb_ham*>(hams, hams + n_sys).size() != (size_t)n_sys) {
+        for (int i = 0; i < n_sys; ++i)
+            QSB_TRY(qsb_ham_apply(hams[i], dtype, 0, nb[i], psi[i], hpsi[i], 0.0, 0.0, 0.0, stream));
+        return QSB_OK;
     }
     if (!qsb::autotune_enabled()) return apply_batched(dtype, n_sys, hams, nb, psi, hpsi, s);
     // autotuner: on the first call for this set of shapes, time the batched form

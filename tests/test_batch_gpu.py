@@ -107,3 +107,18 @@ def test_f32_batch_equals_per_system_apply_bit_for_bit(qsb):
     for H, p, g in zip(hams, psis, got):
         assert torch.equal(H.apply(p, torch.empty_like(p)).view(torch.int32), g.view(torch.int32))
     assert qsb.device_status() == 0
+
+
+def test_one_operator_listed_twice(qsb):
+    """Two bundles under the same operator, the second larger: both results are its own."""
+    import torch
+    systems = _systems(qsb, n_sys=2, seed=6)
+    H, G = systems[0][0], systems[1][0]
+    a = torch.from_numpy(systems[0][1]).cuda()
+    b = torch.cat([a * 2.0, a + 0.5])
+    c = torch.from_numpy(systems[1][1]).cuda()
+    got = [torch.empty_like(p) for p in (a, c, b)]
+    qsb.apply_batch([H, G, H], [a, c, b], got)
+    for K, p, g in ((H, a, got[0]), (G, c, got[1]), (H, b, got[2])):
+        want = K.apply(p, torch.empty_like(p)).cpu().numpy()
+        assert _rel(g.cpu().numpy(), want) < 1e-12
