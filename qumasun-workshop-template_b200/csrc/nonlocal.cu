@@ -658,7 +658,7 @@ nl_apply_kernel(const int* __restrict__ cov_grid, int n_cov, const int* __restri
 // lanes lie in different spheres), and hpsi moves at 5.0 TB/s (FP64) and 3.2 TB/s
 // (FP32) of the 6.4 a plain read-modify-write reaches.
 // 144^3 x 384 FP32 bands, 54 atoms: 3.37 -> 2.87 ms; 96^3 x 128 bands, 16 atoms:
-// FP32 0.311 -> 0.284, FP64 0.384 -> 0.366 ms.  As FP64 tensor-core products (one
+// FP32 0.311 -> 0.284, FP64 0.384 -> 0.363 ms.  As FP64 tensor-core products (one
 // coefficient load per 4 x 8 of them) it took 3.08 and 0.456 ms: the accumulator's
 // layout splits every 256-byte row of hpsi into 64-byte pieces.
 // ---------------------------------------------------------------------------
