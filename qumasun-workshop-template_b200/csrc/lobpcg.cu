@@ -524,25 +524,29 @@ __global__ void pencil_state(const double* __restrict__ A, const double* __restr
     }
     if (bad) atomicOr(state, bad);
 }
+// the pencil (diag(1, 2, ...), identity) in place of one with a state
+__global__ void pencil_replace(double* __restrict__ A, double* __restrict__ B, size_t n, size_t dstep,
+                               const int* __restrict__ state) {
+    if (*state == 0) return;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        A[i] = i % dstep == 0 ? (double)(i / dstep + 1) : 0.0;
+        B[i] = i % dstep == 0 ? 1.0 : 0.0;
+    }
+}
 
 // generalized eigenproblem Sa c = lambda Sb c (m x m), eigenvalues ascending into
 // es->W, eigenvectors into Sa (B-orthonormal).
 qsb_status solve_pencil(qsb_eigensolver* es, int m, cudaStream_t s) {
     // The library's solvers may never come back from a pencil with an entry that is not finite
     // (observed: from one of zeros, whose reduction divides by zero): such a pencil is refused,
-    // one with a vanishing column of B is not positive definite.
-    {
-        const size_t c2 = es->cplx ? 2 : 1, cnt = (size_t)m * m * c2;
-        int state = 0;
-        QSB_CUDA_TRY(cudaMemsetAsync(es->info + 1, 0, sizeof(int), s));
-        pencil_state<<<(int)std::min<size_t>((cnt + 255) / 256, 512), 256, 0, s>>>(es->Sa, es->Sb, cnt,
-                                                                                  ((size_t)m + 1) * c2, es->info + 1);
-        QSB_CUDA_TRY(cudaGetLastError());
-        QSB_CUDA_TRY(cudaMemcpyAsync(&state, es->info + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-        QSB_CUDA_TRY(cudaStreamSynchronize(s));
-        if (state & 1) return fail(QSB_ERR_NUMERIC, "eigensolver: non-finite pencil");
-        if (state & 2) return fail(QSB_ERR_SOLVER, "eigensolver: generalized eigenproblem failed (overlap matrix not positive definite)");
-    }
+    // one with a vanishing column of B is not positive definite.  Both are told by the wait for
+    // the solve's info; until then the solve runs on a pencil put in its place.
+    const size_t c2 = es->cplx ? 2 : 1, cnt = (size_t)m * m * c2, dstep = ((size_t)m + 1) * c2;
+    const int look = (int)std::min<size_t>((cnt + 255) / 256, 512);
+    QSB_CUDA_TRY(cudaMemsetAsync(es->info + 1, 0, sizeof(int), s));
+    pencil_state<<<look, 256, 0, s>>>(es->Sa, es->Sb, cnt, dstep, es->info + 1);
+    pencil_replace<<<look, 256, 0, s>>>(es->Sa, es->Sb, cnt, dstep, es->info + 1);
+    QSB_CUDA_TRY(cudaGetLastError());
     int lwork = 0;
     if (es->cplx) {
         QSB_SOLVER_TRY(cusolverDnZhegvd_bufferSize(es->sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR,
@@ -568,9 +572,13 @@ qsb_status solve_pencil(qsb_eigensolver* es, int m, cudaStream_t s) {
         QSB_SOLVER_TRY(cusolverDnDsygvd(es->sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, m,
                                         es->Sa, m, es->Sb, m, es->W, (double*)es->swork, lwork, es->info));
     }
-    int info = 0;
-    QSB_CUDA_TRY(cudaMemcpyAsync(&info, es->info, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int words[2] = {0, 0};
+    QSB_CUDA_TRY(cudaMemcpyAsync(words, es->info, sizeof(words), cudaMemcpyDeviceToHost, s));
     QSB_CUDA_TRY(cudaStreamSynchronize(s));
+    const int info = words[0];
+    if (words[1] & 1) return fail(QSB_ERR_NUMERIC, "eigensolver: non-finite pencil");
+    if (words[1] & 2)
+        return fail(QSB_ERR_SOLVER, "eigensolver: generalized eigenproblem failed (overlap matrix not positive definite)");
     if (info != 0)
         return fail(QSB_ERR_SOLVER, "eigensolver: generalized eigenproblem failed, info = " + std::to_string(info) +
                                         (info > m ? " (overlap matrix not positive definite)" : ""));
