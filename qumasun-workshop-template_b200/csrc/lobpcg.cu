@@ -513,14 +513,15 @@ qsb_status gram_block(qsb_eigensolver* es, const double* U, const double* V, int
 }
 
 // state |= 1: an entry of the pencil (n doubles each) is not finite, 2: a diagonal entry of
-// B (every dstep-th) is not positive
+// B (every dstep-th) is not positive (B null: a matrix A alone, looked over for 1)
 __global__ void pencil_state(const double* __restrict__ A, const double* __restrict__ B, size_t n, size_t dstep,
                              int* __restrict__ state) {
     int bad = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const double a = A[i], b = B[i];
-        if (!isfinite(a) || !isfinite(b)) bad |= 1;
-        if (i % dstep == 0 && !(b > 0.0)) bad |= 2;
+        if (!isfinite(A[i])) bad |= 1;
+        if (!B) continue;
+        if (!isfinite(B[i])) bad |= 1;
+        if (i % dstep == 0 && !(B[i] > 0.0)) bad |= 2;
     }
     if (bad) atomicOr(state, bad);
 }
@@ -530,23 +531,28 @@ __global__ void pencil_replace(double* __restrict__ A, double* __restrict__ B, s
     if (*state == 0) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         A[i] = i % dstep == 0 ? (double)(i / dstep + 1) : 0.0;
-        B[i] = i % dstep == 0 ? 1.0 : 0.0;
+        if (B) B[i] = i % dstep == 0 ? 1.0 : 0.0;
     }
+}
+
+// The library's dense solvers may never come back from entries that are not finite (observed:
+// from a pencil of zeros, whose reduction divides by zero): such a pencil is refused, one
+// with a vanishing column of B is not positive definite.  Both are told by the wait for
+// the solve's info (es->info[1]); until then the solve runs on a pencil put in its place.
+qsb_status look_over(qsb_eigensolver* es, int m, double* A, double* B, cudaStream_t s) {
+    const size_t c2 = es->cplx ? 2 : 1, cnt = (size_t)m * m * c2, dstep = ((size_t)m + 1) * c2;
+    const int grid = (int)std::min<size_t>((cnt + 255) / 256, 512);
+    QSB_CUDA_TRY(cudaMemsetAsync(es->info + 1, 0, sizeof(int), s));
+    pencil_state<<<grid, 256, 0, s>>>(A, B, cnt, dstep, es->info + 1);
+    pencil_replace<<<grid, 256, 0, s>>>(A, B, cnt, dstep, es->info + 1);
+    QSB_CUDA_TRY(cudaGetLastError());
+    return QSB_OK;
 }
 
 // generalized eigenproblem Sa c = lambda Sb c (m x m), eigenvalues ascending into
 // es->W, eigenvectors into Sa (B-orthonormal).
 qsb_status solve_pencil(qsb_eigensolver* es, int m, cudaStream_t s) {
-    // The library's solvers may never come back from a pencil with an entry that is not finite
-    // (observed: from one of zeros, whose reduction divides by zero): such a pencil is refused,
-    // one with a vanishing column of B is not positive definite.  Both are told by the wait for
-    // the solve's info; until then the solve runs on a pencil put in its place.
-    const size_t c2 = es->cplx ? 2 : 1, cnt = (size_t)m * m * c2, dstep = ((size_t)m + 1) * c2;
-    const int look = (int)std::min<size_t>((cnt + 255) / 256, 512);
-    QSB_CUDA_TRY(cudaMemsetAsync(es->info + 1, 0, sizeof(int), s));
-    pencil_state<<<look, 256, 0, s>>>(es->Sa, es->Sb, cnt, dstep, es->info + 1);
-    pencil_replace<<<look, 256, 0, s>>>(es->Sa, es->Sb, cnt, dstep, es->info + 1);
-    QSB_CUDA_TRY(cudaGetLastError());
+    QSB_TRY(look_over(es, m, es->Sa, es->Sb, s));
     int lwork = 0;
     if (es->cplx) {
         QSB_SOLVER_TRY(cusolverDnZhegvd_bufferSize(es->sol, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR,
@@ -798,7 +804,9 @@ qsb_status ensure_swork(qsb_eigensolver* es, size_t bytes) {
 }
 
 // Hermitian / symmetric eigendecomposition in place (ascending eigenvalues in w)
-qsb_status dense_evd(qsb_eigensolver* es, int k, double* A, int lda, double* w, cudaStream_t s) {
+qsb_status dense_evd(qsb_eigensolver* es, int k, double* A, double* w, cudaStream_t s) {
+    const int lda = k;
+    QSB_TRY(look_over(es, k, A, nullptr, s));
     int lwork = 0;
     if (es->cplx) {
         QSB_SOLVER_TRY(cusolverDnZheevd_bufferSize(es->sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, k,
@@ -813,9 +821,11 @@ qsb_status dense_evd(qsb_eigensolver* es, int k, double* A, int lda, double* w, 
         QSB_SOLVER_TRY(cusolverDnDsyevd(es->sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, k, A, lda, w,
                                         (double*)es->swork, lwork, es->info));
     }
-    int info = 0;
-    QSB_CUDA_TRY(cudaMemcpyAsync(&info, es->info, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int words[2] = {0, 0};
+    QSB_CUDA_TRY(cudaMemcpyAsync(words, es->info, sizeof(words), cudaMemcpyDeviceToHost, s));
     QSB_CUDA_TRY(cudaStreamSynchronize(s));
+    const int info = words[0];
+    if (words[1] & 1) return fail(QSB_ERR_NUMERIC, "eigensolver: non-finite pencil");
     if (info != 0) return fail(QSB_ERR_SOLVER, "eigensolver: dense eigendecomposition failed, info = " + std::to_string(info));
     return QSB_OK;
 }
@@ -873,7 +883,7 @@ qsb_status solve_pencil_overlap_basis(qsb_eigensolver* es, int m, int nout, cuda
         QSB_CUDA_TRY(cudaMemcpyAsync(es->Sb, tmp, sizeof(double) * mm, cudaMemcpyDeviceToDevice, s));
     }
     ++es->last_svqb;
-    QSB_TRY(dense_evd(es, m, es->Sb, m, lam, s));
+    QSB_TRY(dense_evd(es, m, es->Sb, lam, s));
     std::vector<double> hl(m);
     QSB_CUDA_TRY(cudaMemcpyAsync(hl.data(), lam, sizeof(double) * m, cudaMemcpyDeviceToHost, s));
     QSB_CUDA_TRY(cudaStreamSynchronize(s));
@@ -891,7 +901,7 @@ qsb_status solve_pencil_overlap_basis(qsb_eigensolver* es, int m, int nout, cuda
     QSB_CUDA_TRY(cudaGetLastError());
     QSB_TRY(small_gemm(es, false, m, k, m, es->Sa, m, Wm, m, tmp, m));   // A Wm
     QSB_TRY(small_gemm(es, true, k, k, m, Wm, m, tmp, m, Ah, k));        // Wm^H A Wm
-    QSB_TRY(dense_evd(es, k, Ah, k, es->W, s));
+    QSB_TRY(dense_evd(es, k, Ah, es->W, s));
     QSB_TRY(small_gemm(es, false, m, nout, k, Wm, m, Ah, k, tmp, m));    // Wm Y
     rows_scale<<<dim3((m + 127) / 128, nout), 128, 0, s>>>(tmp, d, m, nout, es->cplx, es->Sa);
     QSB_CUDA_TRY(cudaGetLastError());

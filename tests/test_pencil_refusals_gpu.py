@@ -41,11 +41,15 @@ def test_vanishing_directions_are_dropped(qsb, cplx, n, prec):
 
 
 @pytest.mark.parametrize("n", [8, 40])
-def test_a_pencil_of_nan_is_refused(qsb, n):
-    """Bands without any residual cannot be normalised: NaN directions."""
+@pytest.mark.parametrize("straight", [False, True])
+def test_a_pencil_of_nan_is_refused(qsb, n, straight):
+    """Bands without any residual cannot be normalised: NaN directions.  straight: the
+    overlap basis without the Cholesky route in front of it (another Gram kind)."""
     import torch
     _, X, N, dV = _start(qsb, n, False)
     es = qsb.EigenSolver(N, n, False, "fp64")
+    if straight:
+        es.set_gram_kind("bf16x3")
 
     class Raw:
         def __init__(self, ptr, shape):
