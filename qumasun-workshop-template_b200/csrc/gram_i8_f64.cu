@@ -482,7 +482,7 @@ size_t gram_f64_i8_own_bytes(int64_t N, int n, size_t scratch) {
     const GfPlan two = plan_gf(N, 2 * n, GF_OWN_BYTES), three = plan_gf(N, 3 * n, GF_OWN_BYTES),
                  have = plan_gf(N, 3 * n, scratch);
     if (have.bytes > 0 && have.cost <= 1.1 * three.cost) return 0;
-    return std::max(two.bytes, three.bytes);
+    return std::max(two.bytes, three.bytes) + 2048;      // plan_gf's reserve: the same plans within these bytes
 }
 
 // A = scale U^T AU and B = scale U^T U (both m x m, full), m = nblk * n columns; *gave_up
