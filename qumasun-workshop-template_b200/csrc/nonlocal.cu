@@ -1183,7 +1183,7 @@ qsb_status nl_project_tables(qsb_dtype dt, const NLDevice& d, int first_table, i
     tabs.n = ntab;
     // The tensor-core form where its rows are full: a complex bundle (the phases once per 32
     // columns instead of once per 8: 48^3 x 24 bands, FP64, 45 -> 27 us) and the forces' four
-    // tables (0.73 against 1.07 ms at 96^3 x 128); one real table fills half of them and runs
+    // tables (0.75 against 1.07 ms at 96^3 x 128); one real table fills half of them and runs
     // faster in the other (0.29 against 0.48 ms).  FP32 applies keep that one's order of sums.
 #define QSB_MMA(T, C) launch_proj_mma_w<T, C>(d, tabs, psi, N, gx_dx, gy_dy, gz_dz, partial, stride, ncol, s)
 #define QSB_VEC(T, C) launch_proj_w<T, C>(d, (const T*)tabs.t[0], nb, psi, N, gx_dx, gy_dy, gz_dz, partial, ncol, s)
